@@ -316,8 +316,10 @@ FFG_DEV_INLINE void col_fwd2_body(const PrimeDev &P, const FourStep &G, const FS
         for (int t = 0; t < 32; t++) x[t] = d[t];
         dft_dif<PI, 5>(x);
         const uint32_t bb = __brev(bl) >> (32 - (RN - 5));
-        uint32_t cur = twm<PI>(P, (uint64_t)n2 * (q + m3 * bb) % G.L * G.mstep);
-        const uint32_t step = twm<PI>(P, ((uint64_t)n2 * m3 << (RN - 5)) % G.L * G.mstep);
+        // n2 < C times a row frequency below R: exponents below L
+        const uint32_t ms = (uint32_t)G.mstep;
+        uint32_t cur = twm<PI>(P, n2 * (q + m3 * bb) * ms);
+        const uint32_t step = twm<PI>(P, (n2 * m3 << (RN - 5)) * ms);
         uint32_t *o = y + (size_t)(32 * b) * C + n2;
 #pragma unroll
         for (int u = 0; u < 32; u++) {

@@ -375,9 +375,12 @@ FFG_DEV_INLINE void tile_digits(uint32_t *__restrict__ smem, uint32_t stride, co
     }
 }
 
-// ω_L^e (e < L, L | M) in Montgomery form, from the two small tables.
+// ω_L^e (e < L, L | M) in Montgomery form, from the two small tables; E =
+// e M / L < M.  The four-step exponents need no reduction modulo L: n2 < C and
+// k1 < R give n2 k1 < L, and 32 bits hold E (a 64-bit modulo here would cost
+// about 70 instructions, two for every 8 to 32 residues of a pass).
 template <int PI>
-FFG_DEV_INLINE uint32_t twm(const PrimeDev &P, uint64_t E) {
+FFG_DEV_INLINE uint32_t twm(const PrimeDev &P, uint32_t E) {
     const uint32_t lo = __ldg(&P.twl[E & (FFG_TW_LO - 1)]);
     const uint32_t hi = __ldg(&P.twh[E >> FFG_TW_LO_LG]);
     return mo<PI>(lo, hi);

@@ -112,8 +112,9 @@ FFG_DEV_INLINE void col_fwd_body(const PrimeDev &P, const FourStep &G, const FSJ
     lines_fwd<PI>(smem, wlg, G.rn, G.r3, stride, P);
     // twiddle ω_L^(n2 k1) for k1 = r0 + m dr: a running Montgomery product
     const uint32_t n2 = c0 + c;
-    uint32_t cur = twm<PI>(P, (uint64_t)n2 * r0 % G.L * G.mstep);
-    const uint32_t step = twm<PI>(P, (uint64_t)n2 * dr % G.L * G.mstep);
+    // r0 and dr may lie past a short column: exponents reduced modulo L
+    uint32_t cur = twm<PI>(P, (uint32_t)((uint64_t)n2 * r0 % G.L * G.mstep));
+    const uint32_t step = twm<PI>(P, (uint32_t)((uint64_t)n2 * dr % G.L * G.mstep));
     uint32_t *y = (op ? J.yb : J.ya) + (size_t)PI * G.L + n2;
     for (uint32_t k1 = r0; k1 < R; k1 += dr) {
         const uint32_t pos = pos_of(k1, G.rn, G.r3);
@@ -184,8 +185,8 @@ FFG_DEV_INLINE void row_body(const PrimeDev &P, const FourStep &G, const FSJob &
     const uint32_t k1 = freq_of(pos, G.rn, G.r3);
     // ω^-e = ω^(M - E); exponents reduced mod L first
     const uint64_t e0 = (uint64_t)threadIdx.x * k1 % G.L * G.mstep, e1 = (uint64_t)kLineThreads * k1 % G.L * G.mstep;
-    uint32_t cur = twm<PI>(P, e0 ? FFG_M - e0 : 0);
-    const uint32_t step = twm<PI>(P, e1 ? FFG_M - e1 : 0);
+    uint32_t cur = twm<PI>(P, (uint32_t)(e0 ? FFG_M - e0 : 0));
+    const uint32_t step = twm<PI>(P, (uint32_t)(e1 ? FFG_M - e1 : 0));
     for (uint32_t i = threadIdx.x; i < C; i += kLineThreads) {
         ya[i] = mo<PI>(fa[pad_idx(i)], cur);
         cur = mo<PI>(cur, step);

@@ -58,9 +58,10 @@ template <int PI>
 struct BackTwiddle {
     uint32_t cur, step;
     FFG_DEV_INLINE BackTwiddle(const PrimeDev &P, const FourStep &G, uint32_t k1, uint32_t n0, uint32_t d) {
-        const uint64_t e0 = (uint64_t)n0 * k1 % G.L * G.mstep, e1 = (uint64_t)d * k1 % G.L * G.mstep;
-        cur = twm<PI>(P, e0 ? FFG_M - e0 : 0);
-        step = twm<PI>(P, e1 ? FFG_M - e1 : 0);
+        // n0, d < C and k1 < R: both exponents below L, their multiples of M / L below M
+        const uint32_t ms = (uint32_t)G.mstep, e0 = n0 * k1 * ms, e1 = d * k1 * ms;
+        cur = twm<PI>(P, e0 ? (uint32_t)FFG_M - e0 : 0);
+        step = twm<PI>(P, e1 ? (uint32_t)FFG_M - e1 : 0);
     }
     FFG_DEV_INLINE uint32_t apply(uint32_t x) {
         const uint32_t r = mo<PI>(x, cur);
