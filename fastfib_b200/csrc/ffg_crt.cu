@@ -1,17 +1,37 @@
 // CRT recombination and the fast-doubling linear passes, for sm_100a.
 //
-// k_crt: one CTA per 2048 coefficients (= 32 * width output limbs exactly).
-//   1. Garner's method per coefficient (the reference's crt_garner8,
-//      src/crt.c:38-64), in parallel, for the block plus a halo of the few
-//      coefficients below it that reach into its limbs:
+// k_crt, k_crt_pair, k_crt_flat (widths 32..35, every plan but the split's
+// narrow ones): one CTA per 2048 coefficients, as 64 super-limbs of 32
+// coefficients, which are exactly b 32-bit words of the product.
+//   1. All 256 threads run Garner's method (the reference's crt_garner8,
+//      src/crt.c:38-64) on quads of coefficients straight from global memory,
 //        x2 = (r2 - r1) p1^-1 mod p2,  x3 = ((r3 - r1) p1^-1 - x2) p2^-1 mod p3,
-//        X  = r1 + x2 p1 + x3 p1 p2  < p1 p2 p3 < 2^93.
+//        X  = r1 + x2 p1 + x3 p1 p2  < p1 p2 p3 < 2^93,
+//      and put the three words of every X into shared memory: 64 rows of 32
+//      coefficients per word, 36 words apart (16-byte accesses without bank
+//      conflicts).
+//   2. Each of 64 threads adds the 32 values of a row, each at its shift (a
+//      compile-time constant: the pattern repeats every 32 coefficients), into a
+//      running 128-bit sum that gives off one 32-bit word a coefficient
+//      (crt_pack64, src/crt.c:70-87, one run per thread).  What is left over
+//      (below 2^64) is the next super-limb's carry-in.
+//   3. With it added, a super-limb generates or propagates single carry bits:
+//      ballots over the warp, maps over the warps (ffg_ripple.cuh), and the
+//      CTA that finishes last settles the bits between CTAs (settle_cta).  A
+//      CTA computes the carry-in at its own lower end from the 4 coefficients
+//      below it: their parts above the boundary and the column sum of the 64
+//      bits below it, which the true carry exceeds by at most one bit.
+// Long products are bound by issue and memory together (at 2^24 coefficients
+// 80 us, 268 MB: 51 % of the copy bandwidth), short ones by latency.  The form
+// this replaces summed, for every limb, the shifted 128-bit slices of the 4 to 5
+// coefficients over it: about 195 instructions a coefficient against 75 here,
+// 147 us at 2^24 coefficients and 13.5 against 10.6 us for one of a few CTAs.
+// k_crt_narrow (the split's widths 8..31): one CTA per 2048 coefficients.
+//   1. Garner per coefficient for the block plus a halo below it.
 //   2. Every limb j sums the slices of the coefficients X_i 2^(i b) that
-//      overlap it (3-6 of them): the column sum lo_j + 2^64 hi_j.  This is the
-//      reference's crt_pack64 (src/crt.c:70-87) with the running carry turned
-//      into per-limb sums.
-//   3. cta_resolve (ffg_ripple.cuh) settles the one-bit ripples; the CTA
-//      that finishes last settles the carries between CTAs (settle_cta).
+//      overlap it: the column sum lo_j + 2^64 hi_j.
+//   3. cta_resolve (ffg_ripple.cuh) settles the one-bit ripples; settle_cta the
+//      carries between CTAs.
 // A small signed constant is added to the product on the way (the final
 // +-2 of fast doubling, src/fib.c:249) in two's complement over the output.
 //
@@ -34,51 +54,11 @@ constexpr uint32_t CRT_HALO_MAX = 24;   // ceil(156 / b) + 1 for b >= 8, rounded
 constexpr uint32_t CRT_NL_MAX = 32 * 35;
 constexpr uint32_t CRT_NL_PER_W = 32;   // limbs per CTA = 32 * width
 
-FFG_DEV_INLINE int64_t floor_div(int64_t a, int64_t b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 FFG_DEV_INLINE int32_t floor_div32(int32_t a, int32_t b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
 FFG_DEV_INLINE uint32_t crt_ctas_dev(uint64_t nlimbs, uint32_t width) {
     const uint64_t NL = (uint64_t)CRT_NL_PER_W * width;
     return (uint32_t)((nlimbs + NL - 1) / NL);
-}
-
-FFG_DEV_INLINE void crt_block(const GarnerConst &K, const CrtJob &J, uint32_t cta);
-
-__global__ void __launch_bounds__(CRT_THREADS) k_crt(GarnerConst K, CrtJob J) { crt_block(K, J, blockIdx.x); }
-
-// Up to two CRTs by value (the doubling step's two squarings): product
-// blockIdx.y, its CTA blockIdx.x.
-struct CrtPair {
-    CrtJob j[2];
-};
-__global__ void __launch_bounds__(CRT_THREADS) k_crt_pair(GarnerConst K, CrtPair P) {
-    const CrtJob &J = P.j[blockIdx.y];
-    if (blockIdx.x >= crt_ctas_dev(J.nlimbs, J.width)) return;
-    crt_block(K, J, blockIdx.x);
-}
-
-// A batch of CRTs: product blockIdx.y, its CTA blockIdx.x (CTAs past the
-// product's own count return at once, all threads together).
-__global__ void __launch_bounds__(CRT_THREADS) k_crt_batch(GarnerConst K, const CrtJob *__restrict__ jobs) {
-    const CrtJob J = jobs[blockIdx.y];
-    if (blockIdx.x >= crt_ctas_dev(J.nlimbs, J.width)) return;
-    crt_block(K, J, blockIdx.x);
-}
-
-// CRTs of any sizes in one launch: CTA b runs CTA b - first[j] of job j,
-// first[j] <= b < first[j + 1] (first: count + 1 prefix sums of the jobs'
-// CTA counts), found by binary search.
-__global__ void __launch_bounds__(CRT_THREADS) k_crt_flat(GarnerConst K, const CrtJob *__restrict__ jobs,
-                                                         const uint32_t *__restrict__ first, uint32_t count) {
-    const uint32_t b = blockIdx.x;
-    uint32_t lo = 0, hi = count; // invariant: first[lo] <= b < first[hi]
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (__ldg(&first[mid]) <= b) lo = mid;
-        else hi = mid;
-    }
-    const CrtJob J = jobs[lo];
-    crt_block(K, J, b - __ldg(&first[lo]));
 }
 
 // Garner's recombination of one coefficient's residues: X < p1 p2 p3 < 2^93.
@@ -94,19 +74,15 @@ FFG_DEV_INLINE u128 garner(const GarnerConst &K, uint32_t r1, uint32_t r2, uint3
 }
 
 // Column sum lo + 2^64 hi of limb j (relative to the CTA's first limb) over
-// the values Z_i 2^(i b) (i relative to the CTA's first coefficient, stored
-// from -halo), every Z_i below 2^(top + 1).  B: the width when known at
-// compile time (0: bw at run time); indices and shifts fit 32 bits (j is at
-// most 32 * 35 limbs, i at most 2048 + halo coefficients).
-template <int B>
-FFG_DEV_INLINE void column_sum_w(const uint64_t *Zlo, const uint32_t *Zhi, int32_t j, uint32_t bw, int32_t halo,
-                                 int32_t top, uint64_t &s_lo, uint32_t &s_hi) {
-    const int32_t b = B ? B : (int32_t)bw;
-    const int32_t ilo = floor_div32(64 * j - top + b - 1, b), ihi = floor_div32(64 * j + 63, b);
+// the values X_i 2^(i b) (i relative to the CTA's first coefficient, stored
+// from -halo), every X_i below 2^93.
+FFG_DEV_INLINE void column_sum(const uint64_t *Xlo, const uint32_t *Xhi, int32_t j, int32_t b, int32_t halo,
+                               uint64_t &s_lo, uint32_t &s_hi) {
+    const int32_t ilo = floor_div32(64 * j - 92 + b - 1, b), ihi = floor_div32(64 * j + 63, b);
     s_lo = 0;
     s_hi = 0;
     for (int32_t i = ilo < -halo ? -halo : ilo; i <= ihi; i++) {
-        const u128 X = ((u128)Zhi[i + halo] << 64) | Zlo[i + halo];
+        const u128 X = ((u128)Xhi[i + halo] << 64) | Xlo[i + halo];
         const int32_t sft = i * b - 64 * j;
         const uint64_t part = sft >= 0 ? (uint64_t)(X << sft) : (uint64_t)(X >> (-sft));
         s_lo += part;
@@ -114,20 +90,8 @@ FFG_DEV_INLINE void column_sum_w(const uint64_t *Zlo, const uint32_t *Zhi, int32
     }
 }
 
-// The same with big_mul_ntt's widths (32..35) as compile-time divisors; b is
-// the same for every thread of a CTA, so the switch does not diverge.
-FFG_DEV_INLINE void column_sum(const uint64_t *Zlo, const uint32_t *Zhi, int32_t j, uint32_t b, int32_t halo,
-                               int32_t top, uint64_t &s_lo, uint32_t &s_hi) {
-    switch (b) {
-    case 32: column_sum_w<32>(Zlo, Zhi, j, b, halo, top, s_lo, s_hi); return;
-    case 33: column_sum_w<33>(Zlo, Zhi, j, b, halo, top, s_lo, s_hi); return;
-    case 34: column_sum_w<34>(Zlo, Zhi, j, b, halo, top, s_lo, s_hi); return;
-    case 35: column_sum_w<35>(Zlo, Zhi, j, b, halo, top, s_lo, s_hi); return;
-    default: column_sum_w<0>(Zlo, Zhi, j, b, halo, top, s_lo, s_hi); return;
-    }
-}
-
-FFG_DEV_INLINE void crt_block(const GarnerConst &K, const CrtJob &J, uint32_t cta) {
+__global__ void __launch_bounds__(CRT_THREADS) k_crt_narrow(GarnerConst K, CrtJob J) {
+    const uint32_t cta = blockIdx.x;
     extern __shared__ __align__(16) unsigned char sm[];
     uint64_t *Xlo = (uint64_t *)sm;                              // CRT_COEF + halo
     uint64_t *lo = Xlo + CRT_COEF + CRT_HALO_MAX;                // NL limbs
@@ -179,7 +143,7 @@ FFG_DEV_INLINE void crt_block(const GarnerConst &K, const CrtJob &J, uint32_t ct
     for (int32_t j = (int32_t)threadIdx.x - 1; j < (int32_t)NL; j += blockDim.x) {
         uint64_t s_lo;
         uint32_t s_hi;
-        column_sum(Xlo, Xhi, j, b, halo, 92, s_lo, s_hi);
+        column_sum(Xlo, Xhi, j, (int32_t)b, halo, s_lo, s_hi);
         // the constant: +add at limb 0, or 2^(64 nlimbs) + add when negative
         const int64_t jabs = (int64_t)j0 + j;
         if (J.add != 0 && jabs >= 0 && (uint64_t)jabs < J.nlimbs) {
@@ -209,6 +173,424 @@ uint32_t crt_ctas(uint64_t nlimbs, uint32_t width) {
     return (uint32_t)((nlimbs + NL - 1) / NL);
 }
 
+// ---------------------------------------------------- widths 32..35
+
+constexpr int CS_T = CRT_COEF / 32;  // super-limbs of a CTA (64), the unit of crt_ctas()
+constexpr int CS_BIG = 256;          // super-limbs of a CTA of a long product
+constexpr uint32_t CS_ROW = 36;      // shared words of a row (32 coefficients' words; the b words of output)
+// shared words of one word of every value of T super-limbs
+template <int T> __host__ __device__ constexpr uint32_t cs_plane() { return T * CS_ROW; }
+
+// Garner's X as words x[0] + 2^32 x[1] + 2^64 x[2].
+FFG_DEV_INLINE u128 garner_lean(const GarnerConst &K, uint32_t r1, uint32_t r2, uint32_t r3) {
+    const uint32_t p1 = K.p[0], p2 = K.p[1], p3 = K.p[2];
+    const uint32_t x2 = shoup(r2 - min(r1, r1 - p2) + p2, K.i12, K.i12s, p2);
+    const uint32_t t3 = shoup(r3 - min(r1, r1 - p3) + p3, K.i13, K.i13s, p3);
+    const uint32_t x3 = shoup(t3 - min(x2, x2 - p3) + p3, K.i23, K.i23s, p3);
+    // below 2^62, then below 2^64: no carries between the three products
+    const uint64_t lo = (uint64_t)x2 * p1 + r1;
+    const uint64_t t0 = (uint64_t)x3 * (uint32_t)K.p12 + lo;
+    const uint64_t t1 = (uint64_t)x3 * (uint32_t)(K.p12 >> 32) + (t0 >> 32);
+    return ((u128)t1 << 32) | (uint32_t)t0;
+}
+
+FFG_DEV_INLINE uint32_t quad_word(const uint4 &v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
+
+// The carry into the boundary above coefficients x[0..3] (x[3] next below it),
+// short of the single bit that may ripple through the 64 bits below it: the
+// parts of x[3], x[2] above the boundary plus the carries of those 64 bits'
+// column sum (all: a constant limb 2^64 - 1 is part of it).
+template <int B> FFG_DEV_INLINE uint64_t boundary_carry(const u128 (&x)[4], bool all) {
+    u128 s = (u128)(uint64_t)(x[3] << (64 - B)) + (uint64_t)(x[2] >> (2 * B - 64)) + (uint64_t)(x[1] >> (3 * B - 64)) +
+             (uint64_t)(x[0] >> (4 * B - 64));
+    if (all) s += ~0ull;
+    return (uint64_t)(x[3] >> B) + (uint64_t)(x[2] >> (2 * B)) + (uint64_t)(s >> 64);
+}
+
+// A thread's super-limb: words 0..3 in registers, words 4 .. b - 1 in its row.
+struct Super {
+    uint64_t w01, w23;
+    uint32_t ones;  // the and of words 4 .. b - 1
+    uint64_t left;  // carried on into the next super-limb
+    uint64_t bound; // boundary_carry of its last four coefficients
+};
+
+// Sums the 32 values of a row (its three planes).  The words are stored over the
+// values' own low words, always behind the chunk read ahead (chunk c + 1 is
+// loaded before chunk c's words are stored; b words for 32 never overtake it).
+// eval(a, b, c): the value of a coefficient from its words in the three planes
+// (a value's own words, or residues not yet recombined).
+template <int T, int B, class Eval> FFG_DEV_INLINE void super_sum(Super &S, uint32_t *row, bool all, Eval value) {
+    u128 acc = 0, last[4];
+    uint32_t w[4], buf[4];
+    S.ones = ~0u;
+    struct Raw {
+        uint4 r[3];
+    } cur, nxt;
+    auto load = [&](int c, Raw &q) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) q.r[k] = *(const uint4 *)(row + k * cs_plane<T>() + 4 * c);
+    };
+    auto eval = [&](const Raw &q, int e) { return value(quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e)); };
+    load(0, cur);
+    // a chunk at compile-time position c (only width 32 shifts all chunks alike)
+    auto chunk = [&](int c, const Raw &raw) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int i = 4 * c + e, wi = i * B / 32, n = (i + 1) * B / 32 - wi;
+            last[e] = eval(raw, e);
+            acc += last[e] << (i * B % 32);
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                if (m >= n) continue;
+                const uint32_t word = (uint32_t)acc;
+                acc >>= 32;
+                const int at = wi + m;
+                if (at < 4) w[at & 3] = word;
+                else {
+                    S.ones &= word;
+                    buf[at & 3] = word;
+                    if ((at & 3) == 3) *(uint4 *)(row + at - 3) = make_uint4(buf[0], buf[1], buf[2], buf[3]);
+                }
+            }
+        }
+    };
+    load(1, nxt);
+    chunk(0, cur);
+    if (B == 32) {
+#pragma unroll 1
+        for (int c = 1; c < 8; c++) {
+            cur = nxt;
+            if (c < 7) load(c + 1, nxt);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                last[e] = eval(cur, e);
+                acc += last[e];
+                buf[e] = (uint32_t)acc;
+                acc >>= 32;
+                S.ones &= buf[e];
+            }
+            *(uint4 *)(row + 4 * c) = make_uint4(buf[0], buf[1], buf[2], buf[3]);
+        }
+    } else {
+#pragma unroll
+        for (int c = 1; c < 8; c++) {
+            cur = nxt;
+            if (c < 7) load(c + 1, nxt);
+            chunk(c, cur);
+        }
+#pragma unroll
+        for (int m = 0; m < B % 4; m++) row[(B & ~3) + m] = buf[m];
+    }
+    S.w01 = (uint64_t)w[1] << 32 | w[0];
+    S.w23 = (uint64_t)w[3] << 32 | w[2];
+    S.left = (uint64_t)acc;
+    S.bound = boundary_carry<B>(last, all);
+}
+
+FFG_DEV_INLINE u128 words_value(uint32_t a, uint32_t b, uint32_t c) { return (u128)c << 64 | (uint64_t)b << 32 | a; }
+
+// Adds v to words 4 .. b - 1 (v = 1 or -1, a carry or a borrow out of the words
+// below): rare.  Returns the carry or borrow out of the super-limb.
+template <int B> FFG_DEV_INLINE bool super_ripple(Super &S, uint32_t *row, uint32_t v) {
+    bool on = true;
+    uint32_t ones = ~0u;
+    for (int k = 4; k < B; k++) {
+        uint32_t x = row[k];
+        if (on) {
+            on = v == 1 ? x == ~0u : x == 0;
+            x += v;
+            row[k] = x;
+        }
+        ones &= x;
+    }
+    S.ones = ones;
+    return on;
+}
+
+// What the threads of a CTA share while carries are resolved.
+struct SuperShared {
+    uint64_t left[CS_BIG];
+    uint32_t gG[CS_BIG / 32], gP[CS_BIG / 32];
+    uint64_t bound;
+};
+
+// Resolves the CTA's super-limbs (thread t < T its t-th) assuming no carry
+// bit comes into the CTA, and stores words 0..3 to the rows; thread 0 gets the
+// CTA's carry map.  All threads call it.  cin: the first super-limb's carry-in
+// (the others' is their neighbour's left).  sub > 0: the constant is -sub in the
+// first limb's super-limb (1 in the others), in two's complement over the whole
+// number.
+template <int T, int B>
+FFG_DEV_INLINE uint32_t super_resolve(Super &S, uint32_t *row, SuperShared &sh, uint64_t cin, uint64_t sub) {
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    constexpr uint32_t NW = T / 32;
+    const bool mine = t < T;
+    if (mine) {
+        if (sub) { // plus 2^(32 b) - sub
+            bool br = S.w01 < sub;
+            S.w01 -= sub;
+            if (br) {
+                br = S.w23 == 0;
+                S.w23 -= 1;
+                if (br) br = super_ripple<B>(S, row, ~0u);
+            }
+            S.left += !br;
+        }
+        sh.left[t] = S.left;
+        if (t == T - 1) sh.bound = S.bound;
+    }
+    __syncthreads();
+    uint32_t Gm = 0, Pm = 0;
+    if (mine) {
+        const uint64_t h = t ? sh.left[t - 1] : cin;
+        bool G = false;
+        S.w01 += h;
+        if (S.w01 < h) {
+            S.w23 += 1;
+            if (S.w23 == 0) G = super_ripple<B>(S, row, 1);
+        }
+        const bool P = !G && (S.w01 & S.w23) == ~0ull && S.ones == ~0u;
+        Gm = __ballot_sync(0xffffffffu, G), Pm = __ballot_sync(0xffffffffu, P);
+        if (lane == 0) {
+            sh.gG[warp] = Gm;
+            sh.gP[warp] = Pm;
+        }
+    }
+    __syncthreads();
+    uint32_t c0 = 0, c1 = 1, cw = 0; // carries out of the warps so far, for carry-in 0 and 1
+    if (mine) {
+#pragma unroll
+        for (uint32_t k = 0; k < NW; k++) {
+            if (k == warp) cw = c0;
+            const uint32_t m = map_of_group(sh.gG[k], sh.gP[k]);
+            c0 = map_apply(m, c0);
+            c1 = map_apply(m, c1);
+        }
+        const uint64_t A = Gm | Pm, Bm = Gm;
+        if ((((uint32_t)((A + Bm + cw) ^ A ^ Bm)) >> lane) & 1u) {
+            if (++S.w01 == 0 && ++S.w23 == 0) super_ripple<B>(S, row, 1);
+        }
+        *(uint4 *)row = make_uint4((uint32_t)S.w01, (uint32_t)(S.w01 >> 32), (uint32_t)S.w23, (uint32_t)(S.w23 >> 32));
+    }
+    // the carry out of the CTA, less what the next CTA finds by itself: 0 or 1
+    const uint32_t d = (uint32_t)(sh.left[T - 1] - sh.bound);
+    __syncthreads();
+    return (d + c0) | ((d + c1) << 1);
+}
+
+// The CTA's words (rows of b) to its T b / 2 limbs from j0 of out, below nlimbs.
+template <int T, int B> FFG_DEV_INLINE void super_store(const uint32_t *rows, uint64_t *out, uint64_t j0, uint64_t nlimbs) {
+    const uint32_t nl = T * B / 2;
+    const uint32_t lim = nlimbs > j0 ? (nlimbs - j0 < nl ? (uint32_t)(nlimbs - j0) : nl) : 0;
+    for (uint32_t l = threadIdx.x; l < lim; l += blockDim.x) {
+        const uint32_t k = 2 * l, r = k / B, c = k - r * B;
+        uint64_t v;
+        if (B % 2 == 0) {
+            v = *(const uint64_t *)(rows + r * CS_ROW + c);
+        } else {
+            const uint32_t lo = rows[r * CS_ROW + c];
+            const uint32_t hi = c + 1 < B ? rows[r * CS_ROW + c + 1] : rows[(r + 1) * CS_ROW];
+            v = (uint64_t)hi << 32 | lo;
+        }
+        out[j0 + l] = v;
+    }
+}
+
+// What a CTA shares besides its planes: the values of the 4 coefficients below it.
+struct CrtShared {
+    alignas(16) uint32_t halo[2][3][4];
+    SuperShared sup;
+};
+FFG_DEV_INLINE void halo_value(const uint32_t (&h)[3][4], u128 (&x)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) x[e] = (u128)h[2][e] << 64 | (uint64_t)h[1][e] << 32 | h[0][e];
+}
+
+// Residues of the CTA's coefficients (and of the 4 below it) into three planes,
+// zero at or past conv (Garner of zeros is zero): cp.async, so that a CTA's loads
+// are all in flight at once without a register each.
+template <int T>
+FFG_DEV_INLINE void super_stage(uint32_t *planes, uint32_t (&halo)[3][4], const uint32_t *y, uint64_t stride,
+                                int64_t ibase, uint64_t conv) {
+    auto copy = [&](uint32_t *dst, const uint32_t *src, int64_t gi) {
+        const uint32_t n = gi >= 0 && (uint64_t)gi < conv ? (conv - gi < 4 ? (uint32_t)(conv - gi) * 4 : 16u) : 0u;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(src + (n ? gi : 0)), "r"(n)
+                     : "memory");
+    };
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+#pragma unroll
+        for (uint32_t v = 0; v < 8; v++) {
+            const uint32_t q = threadIdx.x + v * T;
+            copy(planes + k * cs_plane<T>() + (q >> 3) * CS_ROW + (q & 7) * 4, y + k * stride, ibase + 4 * (int64_t)q);
+        }
+        if (threadIdx.x == T - 1) copy(halo[k], y + k * stride, ibase - 4);
+    }
+}
+FFG_DEV_INLINE void super_staged() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+}
+
+// Values of the CTA's coefficients into the planes: ld(gi) loads the residues
+// of coefficients gi .. gi + 3, eval(raw, e, z) gives the values of the e-th.
+// A thread's loads are issued before any arithmetic; lanes 0..3 of the last
+// warp also do one coefficient each of the 4 below the CTA.
+template <int NT, int NO, class Raw, class Ld, class Eval>
+FFG_DEV_INLINE void super_fill(uint32_t *planes, CrtShared &sh, int64_t ibase, Ld ld, Eval eval) {
+    constexpr uint32_t PER = CRT_COEF / 4 / NT, AHEAD = NO == 1 ? 2 : 1; // quads a thread, AHEAD loaded at a time
+    const uint32_t t = threadIdx.x, low = t - (NT - 32); // 0..3: a coefficient below the CTA
+    Raw raw[AHEAD], hr;
+    if (low < 4) ld(ibase - 4, hr);
+    auto put = [&](const Raw &r, uint32_t q) {
+        uint32_t x[NO][3][4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            u128 z[NO];
+            eval(r, e, z);
+#pragma unroll
+            for (int k = 0; k < NO; k++)
+#pragma unroll
+                for (int m = 0; m < 3; m++) x[k][m][e] = (uint32_t)(z[k] >> (32 * m));
+        }
+        uint32_t *d = planes + (q >> 3) * CS_ROW + (q & 7) * 4;
+#pragma unroll
+        for (int k = 0; k < NO; k++)
+#pragma unroll
+            for (int m = 0; m < 3; m++)
+                *(uint4 *)(d + (3 * k + m) * cs_plane<CS_T>()) =
+                    make_uint4(x[k][m][0], x[k][m][1], x[k][m][2], x[k][m][3]);
+    };
+#pragma unroll 1
+    for (uint32_t v0 = 0; v0 < PER; v0 += AHEAD) {
+#pragma unroll
+        for (uint32_t v = 0; v < AHEAD; v++) ld(ibase + 4 * (int64_t)(t + (v0 + v) * NT), raw[v]);
+#pragma unroll
+        for (uint32_t v = 0; v < AHEAD; v++) put(raw[v], t + (v0 + v) * NT);
+    }
+    if (low < 4) {
+        u128 z[NO];
+        eval(hr, (int)low, z);
+#pragma unroll
+        for (int k = 0; k < NO; k++)
+#pragma unroll
+            for (int m = 0; m < 3; m++) sh.halo[k][m][low] = (uint32_t)(z[k] >> (32 * m));
+    }
+    __syncthreads();
+}
+
+struct Raw3 {
+    uint4 r[3];
+};
+// Residues of coefficients gi .. gi + 3 (gi a multiple of 4; the arrays are a
+// multiple of 16 words long), zero at or past conv: Garner of zeros is zero.
+FFG_DEV_INLINE void ld_residues(uint4 *r, const uint32_t *y, uint64_t stride, int64_t gi, uint64_t conv) {
+    const bool in = gi >= 0 && (uint64_t)gi < conv;
+#pragma unroll
+    for (int k = 0; k < 3; k++) r[k] = in ? __ldg((const uint4 *)(y + k * stride + gi)) : make_uint4(0, 0, 0, 0);
+    if (in && (uint64_t)gi + 4 > conv) {
+        const uint32_t n = (uint32_t)(conv - (uint64_t)gi); // 1 .. 3 words
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            if (n < 2) r[k].y = 0;
+            if (n < 3) r[k].z = 0;
+            r[k].w = 0;
+        }
+    }
+}
+
+// T = CS_T: Garner by all NT threads, sums by T of them (short products: a
+// thread recombines 8 coefficients and adds 32; batches).  T = CS_BIG = NT: every
+// thread recombines and adds its own 32 coefficients in one pass with no barrier
+// in between, and there are a quarter of the carry maps; the latency of 32
+// coefficients a thread does not count when the CTAs fill the GPU twice over.
+template <int NT, int T, int B>
+FFG_DEV_INLINE void crt_super(const GarnerConst &K, const CrtJob &J, uint32_t cta, uint32_t *planes, CrtShared &sh) {
+    const uint32_t t = threadIdx.x;
+    const int64_t ibase = (int64_t)cta * (32 * T);
+    uint32_t *const row = planes + t * CS_ROW;
+    const bool neg = J.add < 0;
+    Super S;
+    uint64_t cin = 0;
+    u128 below[4];
+    auto garner = [&](uint32_t a, uint32_t b, uint32_t c) { return garner_lean(K, a, b, c); };
+    if (NT == T) {
+        super_stage<T>(planes, sh.halo[0], J.y, J.y_stride, ibase, J.conv);
+        super_staged();
+        super_sum<T, B>(S, row, neg, garner);
+        if (t == 0) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) below[e] = garner(sh.halo[0][0][e], sh.halo[0][1][e], sh.halo[0][2][e]);
+        }
+    } else {
+        super_fill<NT, 1, Raw3>(
+            planes, sh, ibase, [&](int64_t gi, Raw3 &q) { ld_residues(q.r, J.y, J.y_stride, gi, J.conv); },
+            [&](const Raw3 &q, int e, u128(&x)[1]) {
+                x[0] = garner(quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e));
+            });
+        if (t < T) super_sum<T, B>(S, row, neg, words_value);
+        if (t == 0) halo_value(sh.halo[0], below);
+    }
+    if (t == 0) cin = cta ? boundary_carry<B>(below, neg) : (neg ? 0 : (uint64_t)J.add);
+    const uint64_t sub = neg ? (t == 0 && cta == 0 ? (uint64_t)-J.add : 1) : 0;
+    const uint32_t map = super_resolve<T, B>(S, row, sh.sup, cin, sub);
+    super_store<T, B>(planes, J.out, (uint64_t)cta * (T * B / 2), J.nlimbs);
+    const uint32_t ncta = (uint32_t)((J.nlimbs + T * B / 2 - 1) / (T * B / 2));
+    if (ncta > 1) {
+        if (t == 0) J.maps[cta] = map;
+        if (last_cta(J.ticket, ncta)) {
+            settle_cta(J.out, J.nlimbs, T * B / 2, J.maps, ncta);
+            if (t == 0) *J.ticket = 0;
+        }
+    }
+}
+
+template <int NT, int T> FFG_DEV_INLINE void crt_any(const GarnerConst &K, const CrtJob &J, uint32_t cta) {
+    extern __shared__ __align__(16) uint32_t cs_rows[];
+    __shared__ CrtShared sh;
+    switch (J.width) {
+    case 32: crt_super<NT, T, 32>(K, J, cta, cs_rows, sh); return;
+    case 33: crt_super<NT, T, 33>(K, J, cta, cs_rows, sh); return;
+    case 34: crt_super<NT, T, 34>(K, J, cta, cs_rows, sh); return;
+    default: crt_super<NT, T, 35>(K, J, cta, cs_rows, sh); return;
+    }
+}
+
+template <int T> __global__ void __launch_bounds__(256, T == CS_BIG ? 2 : 3) k_crt(GarnerConst K, CrtJob J) {
+    crt_any<256, T>(K, J, blockIdx.x);
+}
+
+// Up to two CRTs by value (the doubling step's two squarings): product
+// blockIdx.y, its CTA blockIdx.x.
+struct CrtPair {
+    CrtJob j[2];
+};
+__global__ void __launch_bounds__(256, 3) k_crt_pair(GarnerConst K, CrtPair P) {
+    const CrtJob J = blockIdx.y ? P.j[1] : P.j[0];
+    if (blockIdx.x >= crt_ctas_dev(J.nlimbs, J.width)) return;
+    crt_any<256, CS_T>(K, J, blockIdx.x);
+}
+
+// CRTs of any sizes in one launch: CTA b runs CTA b - first[j] of job j,
+// first[j] <= b < first[j + 1] (first: count + 1 prefix sums of the jobs'
+// CTA counts), found by binary search.
+__global__ void __launch_bounds__(128, 6) k_crt_flat(GarnerConst K, const CrtJob *__restrict__ jobs,
+                                                            const uint32_t *__restrict__ first, uint32_t count) {
+    const uint32_t b = blockIdx.x;
+    uint32_t lo = 0, hi = count; // invariant: first[lo] <= b < first[hi]
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (__ldg(&first[mid]) <= b) lo = mid;
+        else hi = mid;
+    }
+    const CrtJob J = jobs[lo];
+    crt_any<128, CS_T>(K, J, b - __ldg(&first[lo]));
+}
+
+static size_t super_smem(uint32_t T, uint32_t outs) { return (size_t)3 * outs * T * CS_ROW * sizeof(uint32_t); }
+
 static size_t crt_smem() {
     return (CRT_COEF + CRT_HALO_MAX) * (8 + 4) + CRT_NL_MAX * (8 + 4) + 3 * (CRT_NL_MAX / 32) * 4;
 }
@@ -217,11 +599,19 @@ static bool g_crt_configured = false;
 
 cudaError_t crt_kernel_load() {
     if (g_crt_configured) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_crt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)crt_smem());
+    cudaError_t e = cudaFuncSetAttribute(k_crt<CS_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
+    if (!e) e = cudaFuncSetAttribute(k_crt<CS_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_BIG, 1));
+    if (!e) e = cudaFuncSetAttribute(k_crt_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
+    if (!e) e = cudaFuncSetAttribute(k_crt_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)crt_smem());
     if (e) return e;
     g_crt_configured = true;
     return cudaSuccess;
 }
+
+// From this many CTAs of 64 super-limbs a product takes CTAs of 256 instead
+// (at 2^22 coefficients, 2049 against 513 CTAs, 32.0 against 25.1 us; below,
+// CTAs of 256 leave SMs idle).
+constexpr uint32_t kCrtBigCtas = 1024;
 
 cudaError_t launch_crt(const Primes3 &P3, const CrtJob &J, cudaStream_t st) {
     (void)P3;
@@ -229,19 +619,21 @@ cudaError_t launch_crt(const Primes3 &P3, const CrtJob &J, cudaStream_t st) {
     if (e0) return e0;
     const uint32_t ncta = crt_ctas(J.nlimbs, J.width);
     prof_begin(PK_CRT, st);
-    k_crt<<<ncta, CRT_THREADS, crt_smem(), st>>>(garner_const(), J);
+    if (J.width < 32) k_crt_narrow<<<ncta, CRT_THREADS, crt_smem(), st>>>(garner_const(), J);
+    else if (ncta <= kCrtBigCtas) k_crt<CS_T><<<ncta, 256, super_smem(CS_T, 1), st>>>(garner_const(), J);
+    else k_crt<CS_BIG><<<(ncta + 3) / 4, 256, super_smem(CS_BIG, 1), st>>>(garner_const(), J);
     prof_end(PK_CRT, st, 12.0 * (double)J.conv + 8.0 * (double)J.nlimbs);
     return cudaGetLastError();
 }
 
 cudaError_t launch_crt_pair(const CrtJob *jobs, uint32_t count, cudaStream_t st) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(k_crt_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)crt_smem());
-        if (e) return e;
-        configured = true;
+    if (count == 1 || jobs[0].width < 32 || jobs[1].width < 32) {
+        cudaError_t e = cudaSuccess;
+        for (uint32_t i = 0; i < count && !e; i++) e = launch_crt(Primes3{}, jobs[i], st);
+        return e;
     }
-    if (count == 1) return launch_crt(Primes3{}, jobs[0], st);
+    cudaError_t e0 = crt_kernel_load();
+    if (e0) return e0;
     CrtPair P;
     P.j[0] = jobs[0];
     P.j[1] = jobs[1];
@@ -249,38 +641,16 @@ cudaError_t launch_crt_pair(const CrtJob *jobs, uint32_t count, cudaStream_t st)
     double bytes = 0;
     for (int i = 0; i < 2; i++) bytes += 12.0 * (double)jobs[i].conv + 8.0 * (double)jobs[i].nlimbs;
     prof_begin(PK_CRT, st);
-    k_crt_pair<<<dim3(n0 > n1 ? n0 : n1, 2), CRT_THREADS, crt_smem(), st>>>(garner_const(), P);
-    prof_end(PK_CRT, st, bytes);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_crt_batch(const CrtJob *d_jobs, uint32_t count, uint32_t max_ctas, cudaStream_t st,
-                             double bytes) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e =
-            cudaFuncSetAttribute(k_crt_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)crt_smem());
-        if (e) return e;
-        configured = true;
-    }
-    if (!count) return cudaSuccess;
-    prof_begin(PK_CRT, st);
-    k_crt_batch<<<dim3(max_ctas, count), CRT_THREADS, crt_smem(), st>>>(garner_const(), d_jobs);
+    k_crt_pair<<<dim3(n0 > n1 ? n0 : n1, 2), 256, super_smem(CS_T, 1), st>>>(garner_const(), P);
     prof_end(PK_CRT, st, bytes);
     return cudaGetLastError();
 }
 
 cudaError_t launch_crt_flat(const CrtJob *d_jobs, const uint32_t *d_first, uint32_t count, uint32_t total_ctas,
                             cudaStream_t st, double bytes) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(k_crt_flat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)crt_smem());
-        if (e) return e;
-        configured = true;
-    }
     if (!count || !total_ctas) return cudaSuccess;
     prof_begin(PK_CRT, st);
-    k_crt_flat<<<total_ctas, CRT_THREADS, crt_smem(), st>>>(garner_const(), d_jobs, d_first, count);
+    k_crt_flat<<<total_ctas, 128, super_smem(CS_T, 1), st>>>(garner_const(), d_jobs, d_first, count);
     prof_end(PK_CRT, st, bytes);
     return cudaGetLastError();
 }
@@ -295,130 +665,84 @@ cudaError_t launch_crt_flat(const CrtJob *d_jobs, const uint32_t *d_first, uint3
 // <= 2 p1 p2 p3 < 2^94 - K) and Z_i < 4 2^93 + 2^94 < 2^96.  Over the N
 // coefficients the CTAs cover, sum_i B 2^(i b) = K 2^(N b) - K: adding the
 // constant gamma_k + K leaves the output plus K 2^(N b), a multiple of
-// 2^(64 len) that falls off the top (N b >= 64 len).  A CTA recombines both
-// squarings' residues of its coefficients and writes one output (short
-// products: twice the CTAs, gridDim.y = 2) or both in turn (long products,
-// where recombining twice costs more than it hides).  The rest is crt_block
-// with values of up to 96 bits, and the CTA that finishes last settles both
-// outputs' carries.
+// 2^(64 len) that falls off the top (N b >= 64 len).  The rest is crt_super
+// with values of up to 96 bits.  kOuts 1: output blockIdx.y alone (short
+// products, where twice the CTAs hide more than recombining twice costs); 2:
+// both outputs from one recombination.
+struct Raw6 {
+    uint4 r[6];
+};
 
-// Z_k of one coefficient gi from its residues in both squarings.
-FFG_DEV_INLINE u128 crt_lin_z(const GarnerConst &K, const CrtLinJob &J, uint32_t k, int64_t gi, u128 X1, u128 X2,
-                              u128 bias) {
-    if (gi < 0) return 0;
-    const uint64_t alpha = (uint64_t)(k ? J.alpha[1] : J.alpha[0]);
-    const int64_t beta = k ? J.beta[1] : J.beta[0];
-    // alpha > 0; beta of either sign, the sum taken mod 2^128 (exact: 0 <= Z < 2^96)
-    const u128 Z = X1 * alpha + bias;
-    return beta >= 0 ? Z + X2 * (uint64_t)beta : Z - X2 * (uint64_t)(-beta);
-}
-
-// kSplit: output blockIdx.y only, every load of the thread issued first
-// (short products: twice the CTAs); else both outputs from one
-// recombination, loads vector by vector (fewer registers, more CTAs per SM).
-template <bool kSplit>
-__global__ void __launch_bounds__(CRT_THREADS) k_crt_lin(GarnerConst K, CrtLinJob J) {
-    extern __shared__ __align__(16) unsigned char sm[];
-    constexpr uint32_t ZN = CRT_COEF + CRT_HALO_MAX, NZ = kSplit ? 1 : 2;
-    uint64_t *Zlo0 = (uint64_t *)sm;                  // NZ x ZN
-    uint64_t *lo = Zlo0 + NZ * ZN;                    // NL limbs
-    uint32_t *Zhi0 = (uint32_t *)(lo + CRT_NL_MAX);   // NZ x ZN
-    uint32_t *hi = Zhi0 + NZ * ZN;                    // NL
-    uint32_t *gG = hi + CRT_NL_MAX, *gP = gG + CRT_NL_MAX / 32, *gin = gP + CRT_NL_MAX / 32;
-    __shared__ uint32_t hiprev_s;
-
-    const uint32_t kb = kSplit ? blockIdx.y : 0, ke = kSplit ? blockIdx.y + 1 : 2;
-    const uint32_t b = J.width, NL = CRT_NL_PER_W * b, cta = blockIdx.x;
-    const int32_t halo = (int32_t)(((159 + b - 1) / b + 1 + 3) & ~3u);
+template <int NT, int B, int kOuts>
+FFG_DEV_INLINE void crt_lin_super(const GarnerConst &K, const CrtLinJob &J, uint32_t *planes, CrtShared &sh) {
+    const uint32_t t = threadIdx.x, cta = blockIdx.x, ncta = gridDim.x;
     const int64_t ibase = (int64_t)cta * CRT_COEF;
-    const u128 bias = ((u128)1 << (94 - b)) * (((u128)1 << b) - 1);
-
-    constexpr int VPT = (CRT_COEF + CRT_HALO_MAX) / 4 / CRT_THREADS + 1;
-    constexpr int VPF = kSplit ? VPT : 1; // vectors whose loads are in flight together
-    const int32_t nvec = ((int32_t)CRT_COEF + halo) / 4;
+    const int k0 = kOuts == 1 ? (int)blockIdx.y : 0;
+    const u128 bias = ((u128)1 << (94 - B)) * (((u128)1 << B) - 1);
+    const uint64_t conv0 = J.conv[0], conv1 = J.conv[1];
+    uint32_t al[kOuts];
+    int32_t be[kOuts];
 #pragma unroll
-    for (int v0 = 0; v0 < VPT; v0 += VPF) {
-        uint4 rv[VPF][2][3];
-#pragma unroll
-        for (int v = 0; v < VPF; v++) {
-            const int32_t t4 = (int32_t)threadIdx.x + (v0 + v) * (int32_t)blockDim.x;
-            const int64_t gi = ibase - halo + 4 * (int64_t)t4;
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const bool in = t4 < nvec && gi >= 0 && (uint64_t)gi < J.conv[q];
-#pragma unroll
-                for (int c = 0; c < 3; c++)
-                    rv[v][q][c] = in ? __ldg((const uint4 *)(J.y[q] + c * J.y_stride + gi)) : make_uint4(0, 0, 0, 0);
-            }
-        }
-#pragma unroll
-        for (int v = 0; v < VPF; v++) {
-            const int32_t t4 = (int32_t)threadIdx.x + (v0 + v) * (int32_t)blockDim.x;
-            if (t4 >= nvec) break;
-            const int64_t gi0 = ibase - halo + 4 * (int64_t)t4;
-            const uint32_t r[2][3][4] = {{{rv[v][0][0].x, rv[v][0][0].y, rv[v][0][0].z, rv[v][0][0].w},
-                                          {rv[v][0][1].x, rv[v][0][1].y, rv[v][0][1].z, rv[v][0][1].w},
-                                          {rv[v][0][2].x, rv[v][0][2].y, rv[v][0][2].z, rv[v][0][2].w}},
-                                         {{rv[v][1][0].x, rv[v][1][0].y, rv[v][1][0].z, rv[v][1][0].w},
-                                          {rv[v][1][1].x, rv[v][1][1].y, rv[v][1][1].z, rv[v][1][1].w},
-                                          {rv[v][1][2].x, rv[v][1][2].y, rv[v][1][2].z, rv[v][1][2].w}}};
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int64_t gi = gi0 + e;
-                u128 X1 = 0, X2 = 0;
-                if (gi >= 0) {
-                    X1 = (uint64_t)gi < J.conv[0] ? garner(K, r[0][0][e], r[0][1][e], r[0][2][e]) : (u128)0;
-                    X2 = (uint64_t)gi < J.conv[1] ? garner(K, r[1][0][e], r[1][1][e], r[1][2][e]) : (u128)0;
-                }
-#pragma unroll
-                for (uint32_t z = 0; z < NZ; z++) {
-                    const u128 Z = crt_lin_z(K, J, kb + z, gi, X1, X2, bias);
-                    Zlo0[z * ZN + 4 * t4 + e] = (uint64_t)Z;
-                    Zhi0[z * ZN + 4 * t4 + e] = (uint32_t)(Z >> 64);
-                }
-            }
-        }
+    for (int k = 0; k < kOuts; k++) {
+        al[k] = (uint32_t)(k0 + k ? J.alpha[1] : J.alpha[0]);
+        be[k] = k0 + k ? J.beta[1] : J.beta[0];
     }
-    __syncthreads();
-
-    const uint64_t j0 = (uint64_t)cta * NL;
-    const uint32_t ncta = gridDim.x;
-    for (uint32_t k = kb; k < ke; k++) {
-        const uint32_t z = k - kb;
-        const uint64_t add = (uint64_t)(k ? J.gamma[1] : J.gamma[0]) + ((uint64_t)1 << (94 - b)); // gamma + K > 0
-        for (int32_t j = (int32_t)threadIdx.x - 1; j < (int32_t)NL; j += blockDim.x) {
-            uint64_t s_lo;
-            uint32_t s_hi;
-            column_sum(Zlo0 + z * ZN, Zhi0 + z * ZN, j, b, halo, 95, s_lo, s_hi);
-            if (cta == 0 && j == 0) {
-                s_lo += add;
-                s_hi += s_lo < add;
-            }
-            if (j < 0) hiprev_s = s_hi;
-            else {
-                lo[j] = s_lo;
-                hi[j] = s_hi;
+    auto eval = [&](const Raw6 &q, int e, u128(&z)[kOuts]) {
+        const u128 x1 = garner_lean(K, quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e));
+        const u128 x2 = garner_lean(K, quad_word(q.r[3], e), quad_word(q.r[4], e), quad_word(q.r[5], e));
+#pragma unroll
+        for (int k = 0; k < kOuts; k++) { // exact mod 2^128, 0 <= z < 2^96
+            const u128 v = x1 * al[k] + bias;
+            z[k] = be[k] >= 0 ? v + x2 * (uint32_t)be[k] : v - x2 * (uint32_t)(-be[k]);
+        }
+    };
+    super_fill<NT, kOuts, Raw6>(
+        planes, sh, ibase,
+        [&](int64_t gi, Raw6 &q) {
+            ld_residues(q.r, J.y[0], J.y_stride, gi, conv0);
+            ld_residues(q.r + 3, J.y[1], J.y_stride, gi, conv1);
+        },
+        eval);
+#pragma unroll
+    for (int k = 0; k < kOuts; k++) {
+        uint32_t *const row = planes + 3 * k * cs_plane<CS_T>() + t * CS_ROW;
+        Super S;
+        uint64_t cin = 0;
+        if (t < CS_T) super_sum<CS_T, B>(S, row, false, words_value);
+        if (t == 0) {
+            if (cta) {
+                u128 x[4];
+                halo_value(sh.halo[k], x);
+                cin = boundary_carry<B>(x, false);
+            } else {
+                cin = (uint64_t)(k0 + k ? J.gamma[1] : J.gamma[0]) + ((uint64_t)1 << (94 - B)); // gamma + K > 0
             }
         }
-        __syncthreads();
-        const uint32_t map = cta_resolve(lo, hi, cta ? hiprev_s : 0, NL, gG, gP, gin);
-        uint64_t *out = k ? J.out[1] : J.out[0];
-        for (uint32_t j = threadIdx.x; j < NL && j0 + j < J.len; j += blockDim.x) out[j0 + j] = lo[j];
-        if (threadIdx.x == 0) J.maps[(size_t)k * ncta + cta] = map;
-        __syncthreads();
+        const uint32_t map = super_resolve<CS_T, B>(S, row, sh.sup, cin, 0);
+        super_store<CS_T, B>(planes + 3 * k * cs_plane<CS_T>(), k0 + k ? J.out[1] : J.out[0], (uint64_t)cta * (CS_T * B / 2), J.len);
+        if (t == 0) J.maps[(size_t)(k0 + k) * ncta + cta] = map;
     }
     if (ncta > 1 && last_cta(J.ticket, ncta * gridDim.y)) {
-        for (int q = 0; q < 2; q++) settle_cta(q ? J.out[1] : J.out[0], J.len, NL, J.maps + (size_t)q * ncta, ncta);
-        if (threadIdx.x == 0) *J.ticket = 0;
+        for (int q = 0; q < 2; q++)
+            settle_cta(q ? J.out[1] : J.out[0], J.len, CS_T * B / 2, J.maps + (size_t)q * ncta, ncta);
+        if (t == 0) *J.ticket = 0;
     }
 }
 
-static size_t crt_lin_smem(bool split) {
-    return (split ? 1 : 2) * (CRT_COEF + CRT_HALO_MAX) * (8 + 4) + CRT_NL_MAX * (8 + 4) + 3 * (CRT_NL_MAX / 32) * 4;
+template <int NT, int kOuts> __global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2) k_crt_lin(GarnerConst K, CrtLinJob J) {
+    extern __shared__ __align__(16) uint32_t cs_rows[];
+    __shared__ CrtShared sh;
+    switch (J.width) {
+    case 32: crt_lin_super<NT, 32, kOuts>(K, J, cs_rows, sh); return;
+    case 33: crt_lin_super<NT, 33, kOuts>(K, J, cs_rows, sh); return;
+    case 34: crt_lin_super<NT, 34, kOuts>(K, J, cs_rows, sh); return;
+    default: crt_lin_super<NT, 35, kOuts>(K, J, cs_rows, sh); return;
+    }
 }
 
-// Products of up to this many CTAs per output run one output per CTA
-// (measured on the F(10^8) and F(10^9) chains).
+// Up to this many CTAs an output, the two outputs go to CTAs of their own
+// (F(10^8): 200 us of CRT in the chain; with every step so 222; F(10^9) 585
+// against 727).
 static uint32_t crt_lin_split_max() {
     static long v = -1;
     if (v < 0) {
@@ -432,20 +756,16 @@ static uint32_t crt_lin_split_max() {
 cudaError_t launch_crt_lin(const CrtLinJob &J, cudaStream_t st) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(k_crt_lin<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)crt_lin_smem(true));
-        if (!e)
-            e = cudaFuncSetAttribute(k_crt_lin<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)crt_lin_smem(false));
+        cudaError_t e = cudaFuncSetAttribute(k_crt_lin<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
+        if (!e) e = cudaFuncSetAttribute(k_crt_lin<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 2));
         if (e) return e;
         configured = true;
     }
     if (J.width < 32 || J.width > 35 || J.alpha[0] <= 0 || J.alpha[1] <= 0) return cudaErrorInvalidValue;
     const uint32_t ncta = crt_ctas(J.len, J.width);
-    const bool split = ncta <= crt_lin_split_max();
     prof_begin(PK_CRT, st);
-    if (split) k_crt_lin<true><<<dim3(ncta, 2), CRT_THREADS, crt_lin_smem(true), st>>>(garner_const(), J);
-    else k_crt_lin<false><<<dim3(ncta, 1), CRT_THREADS, crt_lin_smem(false), st>>>(garner_const(), J);
+    if (ncta <= crt_lin_split_max()) k_crt_lin<256, 1><<<dim3(ncta, 2), 256, super_smem(CS_T, 1), st>>>(garner_const(), J);
+    else k_crt_lin<128, 2><<<dim3(ncta, 1), 128, super_smem(CS_T, 2), st>>>(garner_const(), J);
     prof_end(PK_CRT, st, 12.0 * (double)(J.conv[0] + J.conv[1]) + 16.0 * (double)J.len);
     return cudaGetLastError();
 }

@@ -214,8 +214,6 @@ cudaError_t launch_bit_length(const uint64_t *x, uint64_t n, uint64_t *d_out, cu
 uint32_t crt_ctas(uint64_t nlimbs, uint32_t width); // CTAs (and carry maps) of one CRT
 __host__ __device__ uint32_t school_ctas(uint64_t nlimbs); // CTAs (and carry maps) of one schoolbook product
 // Batches in device arrays: one launch (plus one settle) for all products.
-cudaError_t launch_crt_batch(const CrtJob *d_jobs, uint32_t count, uint32_t max_ctas, cudaStream_t st,
-                             double bytes);
 // CRTs of different sizes in one launch of total_ctas CTAs: d_first holds the
 // count + 1 prefix sums of the jobs' crt_ctas.
 cudaError_t launch_crt_flat(const CrtJob *d_jobs, const uint32_t *d_first, uint32_t count, uint32_t total_ctas,

@@ -94,55 +94,79 @@ FFG_DEV_INLINE uint32_t cta_resolve(uint64_t *lo, const uint32_t *hi, uint32_t h
 }
 
 // Carries between CTAs, settled by the CTA that finishes last (all of its
-// threads): thread t composes the maps of its run of consecutive CTAs, a
-// block-wide scan of those composites gives the carry into every run (carry
-// 0 into the first CTA), and each thread walks its run again adding the
-// carry into the CTAs that receive one: a carry stops at the first limb that
-// does not wrap, almost always the first.  A CTA whose map is the identity
-// has every limb 2^64 - 1 (Barrett and Newton combinations produce long such
-// runs): the carry zeroes it with stores alone.  A carry still running after
-// kSettleWalk limbs of any other CTA is finished by the whole block
-// afterwards, 256 limbs at a time, so no thread walks thousands of dependent
-// loads.
+// threads).  A CTA's map kills (0), propagates (2) or generates (3) a carry, so
+// 32 CTAs are two ballots, like 32 limbs: the warps read the maps 32 at a time
+// (kSettleGroups groups a round, their loads in flight together), one warp
+// scans the groups' maps, and only groups that see a carry are looked at again
+// (carry 0 into the first CTA).  A run of maps per thread, one dependent L2
+// read after the other, took about 35 us for the 8193 CTAs of a 2^24-word CRT
+// with 64 threads.
+// A carry stops at the first limb that does not wrap, almost always the first.
+// A CTA whose map is the identity has every limb 2^64 - 1 (Barrett and Newton
+// combinations produce long such runs): the carry zeroes it with stores alone.
+// A carry still running after kSettleWalk limbs of any other CTA is finished by
+// the whole block afterwards, blockDim.x limbs at a time, so no thread walks
+// thousands of dependent loads.
 // Maps and limbs written by other CTAs are read through L2.
 constexpr uint32_t kSettleWalk = 8;
 constexpr uint32_t kSettleLong = 64;
+constexpr uint32_t kSettleGroups = 64; // groups of 32 CTAs a round
 
 FFG_DEV_INLINE void settle_cta(uint64_t *out, uint64_t nlimbs, uint32_t cta_limbs, const uint32_t *maps,
                                uint32_t ncta) {
-    __shared__ uint32_t wpre[32];
+    __shared__ uint32_t gG[kSettleGroups], gP[kSettleGroups], gin[kSettleGroups];
     __shared__ uint64_t long_j[kSettleLong], long_end[kSettleLong];
     __shared__ uint32_t nlong;
     __shared__ uint64_t first_s;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (threadIdx.x == 0) nlong = 0;
-    const uint32_t per = (ncta + blockDim.x - 1) / blockDim.x;
-    const uint32_t q0 = min(ncta, threadIdx.x * per), q1 = min(ncta, q0 + per);
-    uint32_t run = 2u; // identity: c -> c
-    for (uint32_t q = q0; q < q1; q++) run = map_then(run, __ldcg(&maps[q]));
-    const uint32_t inc = warp_map_scan(run);
-    if (lane == 31) wpre[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        const uint32_t v = warp_map_scan(lane < nw ? wpre[lane] : 2u);
-        __syncwarp();
-        if (lane < nw) wpre[lane] = v;
-    }
-    __syncthreads();
-    uint32_t exc = __shfl_up_sync(0xffffffffu, inc, 1);
-    if (lane == 0) exc = 2u;
-    const uint32_t before = warp ? map_then(wpre[warp - 1], exc) : exc;
-    uint32_t carry = map_apply(before, 0);
-    for (uint32_t q = q0; q < q1; q++) {
-        const uint32_t mq = __ldcg(&maps[q]);
-        if (carry && mq == 2u) {
-            // the identity map: every limb of the CTA is 2^64 - 1, so the
-            // carry turns them all to 0 and goes on (stores only, no search)
-            const uint64_t end = min(nlimbs, (uint64_t)(q + 1) * cta_limbs);
-            for (uint64_t j = (uint64_t)q * cta_limbs; j < end; j++) out[j] = 0;
-        } else if (carry) {
+    uint32_t carry = 0; // into the round's first CTA (warp 0 keeps it)
+    for (uint32_t base = 0; base < ncta; base += 32 * kSettleGroups) {
+        const uint32_t ng = min(kSettleGroups, (ncta - base + 31) / 32);
+        for (uint32_t g0 = warp; g0 < ng; g0 += 8 * nw) {
+            uint32_t m[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) {
+                const uint32_t g = g0 + k * nw, q = base + 32 * g + lane;
+                m[k] = g < ng && q < ncta ? __ldcg(&maps[q]) : 0u;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) {
+                const uint32_t g = g0 + k * nw;
+                const uint32_t G = __ballot_sync(0xffffffffu, m[k] == 3u), P = __ballot_sync(0xffffffffu, m[k] == 2u);
+                if (g < ng && lane == 0) {
+                    gG[g] = G;
+                    gP[g] = P;
+                }
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {
+            for (uint32_t g0 = 0; g0 < ng; g0 += 32) {
+                const uint32_t g = g0 + lane;
+                const uint32_t inc = warp_map_scan(g < ng ? map_of_group(gG[g], gP[g]) : 2u);
+                uint32_t exc = __shfl_up_sync(0xffffffffu, inc, 1);
+                if (lane == 0) exc = 2u;
+                if (g < ng) gin[g] = map_apply(exc, carry);
+                carry = map_apply(__shfl_sync(0xffffffffu, inc, 31), carry);
+            }
+        }
+        __syncthreads();
+        for (uint32_t g = warp; g < ng; g += nw) {
+            const uint32_t G = gG[g], P = gP[g], c = gin[g];
+            if (!(G | c)) continue; // no carry reaches any of the group's CTAs
+            const uint64_t A = G | P, B = G;
+            const uint32_t carries = (uint32_t)((A + B + c) ^ A ^ B);
+            const uint32_t q = base + 32 * g + lane;
+            if (q >= ncta || !((carries >> lane) & 1u)) continue;
             const uint64_t end = min(nlimbs, (uint64_t)(q + 1) * cta_limbs);
             uint64_t j = (uint64_t)q * cta_limbs;
+            if ((P >> lane) & 1u) {
+                // the identity map: every limb of the CTA is 2^64 - 1, so the
+                // carry turns them all to 0 and goes on (stores only, no search)
+                for (; j < end; j++) out[j] = 0;
+                continue;
+            }
             bool running = true;
             for (uint32_t w = 0; w < kSettleWalk && j < end; w++, j++) {
                 const uint64_t v = __ldcg(&out[j]) + 1;
@@ -166,9 +190,8 @@ FFG_DEV_INLINE void settle_cta(uint64_t *out, uint64_t nlimbs, uint32_t cta_limb
                 }
             }
         }
-        carry = map_apply(mq, carry);
+        __syncthreads(); // the groups' words are rewritten
     }
-    __syncthreads();
     // the long carries, one at a time by the whole block: limbs before the
     // first one that is not 2^64 - 1 become 0, that one gains 1
     const uint32_t nl = min(nlong, kSettleLong);
@@ -191,14 +214,19 @@ FFG_DEV_INLINE void settle_cta(uint64_t *out, uint64_t nlimbs, uint32_t cta_limb
 }
 
 // Called by every CTA of a launch after its limbs and map are written:
-// true in the one CTA that takes the last of ncta tickets.
+// true in the one CTA that takes the last of ncta tickets.  The barrier puts
+// every thread's stores before thread 0's fence, which makes them visible to
+// the device (fences are cumulative); the last CTA's fence and barrier put the
+// reads of its other threads after them.
 FFG_DEV_INLINE bool last_cta(uint32_t *ticket, uint32_t ncta) {
     __shared__ bool last;
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == ncta - 1;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == ncta - 1;
+        __threadfence();
+    }
     __syncthreads();
-    if (last) __threadfence();
     return last;
 }
 
