@@ -12,9 +12,10 @@
 //   k_col_fwd  : digits of a column tile -> length-R forward transforms down
 //                the columns -> twiddle ω_L^(n2 k1) -> residues, row-major
 //   k_row_conv : per row: forward length-C transform of both operands,
-//                pointwise product, inverse, twiddle ω_L^-(n2 k1)
-//   k_col_inv  : inverse length-R transforms down the columns, scale by
-//                2^32 / L, natural coefficient order for the CRT
+//                pointwise product, inverse, twiddle ω_L^-(n2 k1), scale by
+//                2^32 / L
+//   k_col_inv  : inverse length-R transforms down the columns, natural
+//                coefficient order for the CRT
 // The reference's top radix-16 passes over column chunks and in-cache
 // sub-blocks (src/ntt_conv.c:158-226) play the same roles on the CPU; here
 // each pass is one HBM round trip of the residues.
@@ -185,7 +186,8 @@ FFG_DEV_INLINE void row_body(const PrimeDev &P, const FourStep &G, const FSJob &
     const uint32_t k1 = freq_of(pos, G.rn, G.r3);
     // ω^-e = ω^(M - E); exponents reduced mod L first
     const uint64_t e0 = (uint64_t)threadIdx.x * k1 % G.L * G.mstep, e1 = (uint64_t)kLineThreads * k1 % G.L * G.mstep;
-    uint32_t cur = twm<PI>(P, (uint32_t)(e0 ? FFG_M - e0 : 0));
+    // with the convolution's scale 2^32 / L
+    uint32_t cur = sh<PI>(twm<PI>(P, (uint32_t)(e0 ? FFG_M - e0 : 0)), make_uint2(G.scl[PI], G.scls[PI]));
     const uint32_t step = twm<PI>(P, (uint32_t)(e1 ? FFG_M - e1 : 0));
     for (uint32_t i = threadIdx.x; i < C; i += kLineThreads) {
         ya[i] = mo<PI>(fa[pad_idx(i)], cur);
@@ -211,16 +213,15 @@ FFG_DEV_INLINE void col_inv_body(const PrimeDev &P, const FourStep &G, const FSJ
     tile_load<8>(smem, stride, J.ya + (size_t)PI * G.L + c0, C, R, wlg);
     __syncthreads();
     lines_inv<PI>(smem, wlg, G.rn, G.r3, stride, P);
-    const uint2 sc = make_uint2(G.scl[PI], G.scls[PI]);
     if (J.yacc) { // overlap-add of a split output piece
         uint32_t *acc = J.yacc + (size_t)PI * J.acc_stride + J.acc_off + c0 + c;
         for (uint32_t n1 = r0; n1 < R; n1 += dr) {
             const size_t at = (size_t)n1 * C;
-            acc[at] = ad<PI>(acc[at], sh<PI>(col[pad_idx(n1)], sc));
+            acc[at] = ad<PI>(acc[at], col[pad_idx(n1)]);
         }
         return;
     }
-    for (uint32_t n1 = r0; n1 < R; n1 += dr) y[(size_t)n1 * C] = sh<PI>(col[pad_idx(n1)], sc);
+    for (uint32_t n1 = r0; n1 < R; n1 += dr) y[(size_t)n1 * C] = col[pad_idx(n1)];
 }
 
 __global__ void __launch_bounds__(kLineThreads, kLineMinBlocks) k_col_inv(Primes3 P3, FourStep G, FSJobs jobs) {

@@ -52,15 +52,17 @@ template <int CLG> struct RowGeo {
     static_assert(T * GB * RB == C && (MA == 0 || T * GA * RA == C), "every word in one group per step");
 };
 
-// ω_L^-(k1 n2) in Montgomery form for n2 = n0 + d t, t = 0, 1, ...: a running
-// product (the inverse four-step twiddle of the generic row pass).
+// ω_L^-(k1 n2) times the convolution's scale (2^32 / L) in Montgomery form for
+// n2 = n0 + d t, t = 0, 1, ...: a running product (the inverse four-step twiddle
+// of the generic row pass).  The scale costs one product a group here, one a
+// residue in the column pass.
 template <int PI>
 struct BackTwiddle {
     uint32_t cur, step;
     FFG_DEV_INLINE BackTwiddle(const PrimeDev &P, const FourStep &G, uint32_t k1, uint32_t n0, uint32_t d) {
         // n0, d < C and k1 < R: both exponents below L, their multiples of M / L below M
         const uint32_t ms = (uint32_t)G.mstep, e0 = n0 * k1 * ms, e1 = d * k1 * ms;
-        cur = twm<PI>(P, e0 ? (uint32_t)FFG_M - e0 : 0);
+        cur = sh<PI>(twm<PI>(P, e0 ? (uint32_t)FFG_M - e0 : 0), make_uint2(G.scl[PI], G.scls[PI]));
         step = twm<PI>(P, e1 ? (uint32_t)FFG_M - e1 : 0);
     }
     FFG_DEV_INLINE uint32_t apply(uint32_t x) {

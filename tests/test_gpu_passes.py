@@ -1,0 +1,59 @@
+"""GPU test of the fixed-shape four-step passes (ffg_rows.cu, ffg_cols.cu) at
+every column length and row length they instantiate, forced by
+ffg_set_geometry: squares and products, one of them with a short operand (most
+rows of its columns are zero), against the product modulo three 64-bit primes
+and modulo 2^128 (a wrong residue changes the product everywhere)."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+PRIMES = (18446744073709551557, 18446744073709551533, 9223372036854775783)
+
+# (columns of 2^rn or 3 2^rn words, rows of 2^c): every rn with rows of 512, every c with columns of 64 or 192
+SHAPES = [(rn, 9) for rn in range(6, 13)] + [(6, c) for c in range(10, 14)] + [(10, 12), (11, 11)]
+
+
+def _check(ff, na, nb, square):
+    rng = np.random.default_rng(na * 7 + nb)
+    a = rng.integers(0, 2**64, na, dtype=np.uint64)
+    b = a if square else rng.integers(0, 2**64, nb, dtype=np.uint64)
+    da = torch.from_numpy(a.view(np.int64)).cuda()
+    db = da if square else torch.from_numpy(b.view(np.int64)).cuda()
+    out = torch.full((na + nb + 1,), -1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    ff.mul_device(out.data_ptr(), da.data_ptr(), na, 64 * na, db.data_ptr(), nb, 64 * nb, square)
+    torch.cuda.synchronize()
+    x, y = ff.limbs_to_int(a), ff.limbs_to_int(b)
+    z = ff.limbs_to_int(out.cpu().numpy().view(np.uint64))
+    assert z.bit_length() <= 64 * (na + nb)
+    for m in PRIMES + (1 << 128,):
+        assert z % m == (x % m) * (y % m) % m, (na, nb, square, m)
+
+
+@pytest.mark.parametrize("r3", [0, 1])
+@pytest.mark.parametrize("rn,c", SHAPES)
+def test_pass_shapes(ff, rn, c, r3):
+    if r3 and rn > 11:
+        pytest.skip("columns of 3 2^12 words do not fit a tile")
+    ff.init(1 << 23)
+    lg = rn + c
+    L = (3 if r3 else 1) << lg
+    hit = 0
+    for wc in (8, 32):
+        try:
+            ff.set_geometry(lg, r3, c, wc)
+        except ff.FfgError:
+            continue  # 32 long columns do not fit shared memory
+        try:
+            # (limbs of a, of b): 32-bit digits, digits of over 32 bits, a short operand
+            for na, nb in ((L // 4 - 3, None), (L // 4 + L // 256, L // 4 - 4), (L // 2 - L // 32, L // 40)):
+                if ff.plan(64 * na, 64 * (nb or na), nb is None)["L"] == L:
+                    _check(ff, na, nb or na, nb is None)
+                    hit += 1
+        finally:
+            ff.set_geometry(lg, r3, 0, 0)
+            ff.load_tuning()
+    assert hit
