@@ -365,9 +365,14 @@ cudaError_t launch_split_forward(const Primes3 &P3, FourStep G, const FSJobs &jo
     prof_end(PK_COL_FWD, st, res + limb_bytes);
     if (e) return e;
     prof_begin(PK_ROW_CONV, st);
-    k_row_conv<<<dim3(G.R, G.nprimes, njobs), 256, sm_row, st>>>(P3, G, jobs);
+    if (g_row2 && row2_ok(G)) {
+        e = launch_row2(P3, G, jobs, njobs, st);
+    } else {
+        k_row_conv<<<dim3(G.R, G.nprimes, njobs), 256, sm_row, st>>>(P3, G, jobs);
+        e = cudaGetLastError();
+    }
     prof_end(PK_ROW_CONV, st, res * 2);
-    return cudaGetLastError();
+    return e;
 }
 
 // One output piece: pairwise sum + inverse row pass, then the inverse column
@@ -383,9 +388,14 @@ cudaError_t launch_split_piece(const Primes3 &P3, FourStep G, const FSJob &job, 
     const uint32_t tiles = (1u << G.c) / G.wc;
     const double res = 3.0 * 4.0 * (double)G.L;
     prof_begin(PK_ROW_CONV, st);
-    k_row_conv<<<dim3(G.R, G.nprimes, 1), 256, sm_row, st>>>(P3, G, one);
+    if (g_row2 && row2_ok(G)) {
+        e = launch_row2(P3, G, one, 1, st);
+    } else {
+        k_row_conv<<<dim3(G.R, G.nprimes, 1), 256, sm_row, st>>>(P3, G, one);
+        e = cudaGetLastError();
+    }
     prof_end(PK_ROW_CONV, st, res * (2.0 * pairs + 1.0));
-    if ((e = cudaGetLastError())) return e;
+    if (e) return e;
     prof_begin(PK_COL_INV, st);
     if (g_col2 && col2_ok(G)) {
         e = launch_col2(false, P3, G, one, 1, st);

@@ -24,9 +24,13 @@
 // 2^14: 16.8 -> 10.7 us; the row passes of the F(10^8) chain 283 -> 228 us).  Long
 // rows are bound by the integer pipes (L = 2^24: 275 -> 269 us, 4 CTAs an SM).
 //
+// The split's row modes run the same steps: ROW_FWD stops after step C and
+// stores the transformed piece in step C's order, ROW_ACC_INV starts from the
+// sum of its pieces' products in that order.
+//
 // It computes the same residues as the generic row pass of ffg_ntt.cu
-// (k_row_conv, mode ROW_CONV): the order of the frequencies between the
-// forward and the inverse differs, but the pointwise product does not care.
+// (k_row_conv): the order of the frequencies between the forward and the
+// inverse differs, but the pointwise product does not care.
 #include "ffg_internal.h"
 #include "ffg_lines.cuh"
 
@@ -106,24 +110,70 @@ FFG_DEV_INLINE void row_fwd_b(uint32_t *__restrict__ s, uint32_t tau, const uint
     }
 }
 
-template <int PI, int CLG, bool SQ>
-FFG_DEV_INLINE void row2_body(const PrimeDev &P, const FourStep &G, uint32_t *ja, const uint32_t *jb, uint32_t *smem) {
+// What k_row2 does with its rows (FourStep::mode and square).
+enum RowKind { RK_SQUARE, RK_PRODUCT, RK_FORWARD, RK_PIECE };
+
+// 16 consecutive words of a residue row (16-byte aligned: the split's pieces
+// lie in the arena).
+FFG_DEV_INLINE void ld16(uint32_t (&x)[16], const uint32_t *p) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint4 v = __ldg((const uint4 *)p + k);
+        x[4 * k] = v.x, x[4 * k + 1] = v.y, x[4 * k + 2] = v.z, x[4 * k + 3] = v.w;
+    }
+}
+
+// The split's output piece m on 16 words of its row: the sum over i + j = m of
+// the transformed pieces' products (src/mul_split.c:62-78); of a square's equal
+// pairs one is computed and doubled.  at: the words' place in a piece.
+template <int PI> FFG_DEV_INLINE void piece_sum(const FSJob &J, size_t at, uint32_t (&acc)[16]) {
+    const uint32_t m = J.m, i0 = m + 1 > J.kb ? m + 1 - J.kb : 0;
+    uint32_t i1 = m < J.ka - 1 ? m : J.ka - 1;
+    if (J.psq) i1 = m ? min(i1, (m - 1) / 2) : 0; // i < j
+    const uint32_t *pa = J.pa + at, *pb = J.pb + at;
+    uint32_t x[16], y[16];
+#pragma unroll
+    for (int t = 0; t < 16; t++) acc[t] = 0;
+    if (!J.psq || m) {
+#pragma unroll 1
+        for (uint32_t i = i0; i <= i1; i++) {
+            ld16(x, pa + i * J.piece_stride);
+            ld16(y, pb + (m - i) * J.piece_stride);
+#pragma unroll
+            for (int t = 0; t < 16; t++) acc[t] = ad<PI>(acc[t], mo<PI>(x[t], y[t]));
+        }
+    }
+    if (!J.psq) return;
+#pragma unroll
+    for (int t = 0; t < 16; t++) acc[t] = ad<PI>(acc[t], acc[t]);
+    if (m % 2 == 0 && m / 2 < J.ka) {
+        ld16(x, pa + (m / 2) * J.piece_stride);
+#pragma unroll
+        for (int t = 0; t < 16; t++) acc[t] = ad<PI>(acc[t], mo<PI>(x[t], x[t]));
+    }
+}
+
+template <int PI, int CLG, int KIND>
+FFG_DEV_INLINE void row2_body(const PrimeDev &P, const FourStep &G, const FSJob &J, uint32_t *smem) {
     using Q = RowGeo<CLG>;
+    constexpr bool TWO = KIND == RK_PRODUCT;
     const uint32_t r = threadIdx.x / Q::T, tau = threadIdx.x % Q::T;
     const uint32_t pos = blockIdx.x * (blockDim.x / Q::T) + r;
     const size_t rowoff = (size_t)PI * G.L + (size_t)pos * Q::C;
-    uint32_t *ya = ja + rowoff;
-    uint32_t *sa = smem + r * (SQ ? 1 : 2) * Q::LS;
+    uint32_t *ya = J.ya + rowoff;
+    uint32_t *sa = smem + r * (TWO ? 2 : 1) * Q::LS;
     uint32_t *sb = sa + Q::LS;
-    const uint2 *twA = P.stw + c_lines.tw_off[(4 + Q::LB) * 6 + Q::LA];
-    const uint2 *twB = P.stw + c_lines.tw_off[4 * 6 + Q::LB];
 
-    row_fwd_a<PI, CLG>(ya, sa, tau, twA);
-    if (!SQ) row_fwd_a<PI, CLG>(jb + rowoff, sb, tau, twA);
-    __syncthreads();
-    row_fwd_b<PI, CLG>(sa, tau, twB);
-    if (!SQ) row_fwd_b<PI, CLG>(sb, tau, twB);
-    __syncthreads();
+    if (KIND != RK_PIECE) {
+        const uint2 *twA = P.stw + c_lines.tw_off[(4 + Q::LB) * 6 + Q::LA];
+        const uint2 *twB = P.stw + c_lines.tw_off[4 * 6 + Q::LB];
+        row_fwd_a<PI, CLG>(ya, sa, tau, twA);
+        if (TWO) row_fwd_a<PI, CLG>(J.yb + rowoff, sb, tau, twA);
+        __syncthreads();
+        row_fwd_b<PI, CLG>(sa, tau, twB);
+        if (TWO) row_fwd_b<PI, CLG>(sb, tau, twB);
+        __syncthreads();
+    }
 
     // step C, the pointwise product and C^-1 on registers
 #pragma unroll 1
@@ -131,29 +181,40 @@ FFG_DEV_INLINE void row2_body(const PrimeDev &P, const FourStep &G, uint32_t *ja
         const uint32_t b = tau + Q::T * k;
         uint32_t x[16];
         uint32_t *d = sa + 16 * b + (b >> 1);
-        if (!SQ) {
-            uint32_t *e = sb + 16 * b + (b >> 1);
-#pragma unroll
-            for (int t = 0; t < 16; t++) x[t] = e[t];
-            dft_dif<PI, 4>(x);
-#pragma unroll
-            for (int t = 0; t < 16; t++) e[t] = x[t]; // read back below by this thread only
-        }
-#pragma unroll
-        for (int t = 0; t < 16; t++) x[t] = d[t];
-        dft_dif<PI, 4>(x);
-        if (SQ) {
-#pragma unroll
-            for (int t = 0; t < 16; t++) x[t] = mo<PI>(x[t], x[t]);
+        if (KIND == RK_PIECE) {
+            piece_sum<PI>(J, rowoff + 16 * b, x);
         } else {
-            const uint32_t *e = sb + 16 * b + (b >> 1);
+            if (TWO) {
+                uint32_t *e = sb + 16 * b + (b >> 1);
 #pragma unroll
-            for (int t = 0; t < 16; t++) x[t] = mo<PI>(x[t], e[t]);
+                for (int t = 0; t < 16; t++) x[t] = e[t];
+                dft_dif<PI, 4>(x);
+#pragma unroll
+                for (int t = 0; t < 16; t++) e[t] = x[t]; // read back below by this thread only
+            }
+#pragma unroll
+            for (int t = 0; t < 16; t++) x[t] = d[t];
+            dft_dif<PI, 4>(x);
+            if (KIND == RK_FORWARD) { // the transformed piece, in the order RK_PIECE reads
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    ((uint4 *)(ya + 16 * b))[t] = make_uint4(x[4 * t], x[4 * t + 1], x[4 * t + 2], x[4 * t + 3]);
+                continue;
+            }
+            if (TWO) {
+                const uint32_t *e = sb + 16 * b + (b >> 1);
+#pragma unroll
+                for (int t = 0; t < 16; t++) x[t] = mo<PI>(x[t], e[t]);
+            } else {
+#pragma unroll
+                for (int t = 0; t < 16; t++) x[t] = mo<PI>(x[t], x[t]);
+            }
         }
         dft_dit<PI, 4>(x);
 #pragma unroll
         for (int t = 0; t < 16; t++) d[t] = x[t];
     }
+    if (KIND == RK_FORWARD) return;
     __syncthreads();
 
     // B^-1
@@ -203,31 +264,28 @@ FFG_DEV_INLINE void row2_body(const PrimeDev &P, const FourStep &G, uint32_t *ja
     }
 }
 
-template <int CLG, bool SQ>
-__global__ void __launch_bounds__(256, CLG == 13 && !SQ ? 3 : 4) k_row2(Primes3 P3, FourStep G, FSJobs jobs) {
+template <int CLG, int KIND>
+__global__ void __launch_bounds__(256, CLG == 13 && KIND == RK_PRODUCT ? 3 : 4) k_row2(Primes3 P3, FourStep G, FSJobs jobs) {
     extern __shared__ uint32_t smem[];
-    __shared__ uint32_t *jy[2];
-    if (threadIdx.x == 0) {
-        const FSJob &J = jobs.ext ? jobs.ext[blockIdx.z] : jobs.j[blockIdx.z < FFG_FS_JOBS ? blockIdx.z : 0];
-        jy[0] = J.ya;
-        jy[1] = J.yb;
-    }
+    __shared__ FSJob J;
+    if (threadIdx.x == 0) J = jobs.ext ? jobs.ext[blockIdx.z] : jobs.j[blockIdx.z < FFG_FS_JOBS ? blockIdx.z : 0];
     __syncthreads();
     switch (blockIdx.y + G.prime0) {
-    case 0: row2_body<0, CLG, SQ>(P3.pr[0], G, jy[0], jy[1], smem); break;
-    case 1: row2_body<1, CLG, SQ>(P3.pr[1], G, jy[0], jy[1], smem); break;
-    default: row2_body<2, CLG, SQ>(P3.pr[2], G, jy[0], jy[1], smem); break;
+    case 0: row2_body<0, CLG, KIND>(P3.pr[0], G, J, smem); break;
+    case 1: row2_body<1, CLG, KIND>(P3.pr[1], G, J, smem); break;
+    default: row2_body<2, CLG, KIND>(P3.pr[2], G, J, smem); break;
     }
 }
 
-template <int CLG, bool SQ>
+template <int CLG, int KIND>
 static cudaError_t launch_row2_t(const Primes3 &P3, const FourStep &G, const FSJobs &jobs, uint32_t njobs,
                                  cudaStream_t st) {
     using Q = RowGeo<CLG>;
-    const size_t smax = (size_t)Q::ROWS * (SQ ? 1 : 2) * Q::LS * sizeof(uint32_t);
+    constexpr uint32_t lines = KIND == RK_PRODUCT ? 2 : 1;
+    const size_t smax = (size_t)Q::ROWS * lines * Q::LS * sizeof(uint32_t);
     static bool attr = false;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_row2<CLG, SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
+        cudaError_t e = cudaFuncSetAttribute(k_row2<CLG, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
         if (e) return e;
         attr = true;
     }
@@ -236,8 +294,8 @@ static cudaError_t launch_row2_t(const Primes3 &P3, const FourStep &G, const FSJ
     uint32_t rows = Q::ROWS;
     while (rows > 1 && (uint64_t)(G.R / rows) * G.nprimes * njobs < 3 * 148) rows >>= 1;
     while (rows > 1 && G.R % rows) rows >>= 1;
-    const size_t sm = (size_t)rows * (SQ ? 1 : 2) * Q::LS * sizeof(uint32_t);
-    k_row2<CLG, SQ><<<dim3(G.R / rows, G.nprimes, njobs), rows * Q::T, sm, st>>>(P3, G, jobs);
+    const size_t sm = (size_t)rows * lines * Q::LS * sizeof(uint32_t);
+    k_row2<CLG, KIND><<<dim3(G.R / rows, G.nprimes, njobs), rows * Q::T, sm, st>>>(P3, G, jobs);
     return cudaGetLastError();
 }
 
@@ -245,18 +303,29 @@ static cudaError_t launch_row2_t(const Primes3 &P3, const FourStep &G, const FSJ
 // own constant bank); set once with the others.
 cudaError_t set_line_consts_rows(const LineConsts &h) { return cudaMemcpyToSymbol(c_lines, &h, sizeof h); }
 
-// Whether the fixed-shape row pass takes this geometry (ROW_CONV rows of
-// 2^9 .. 2^13 words).
-bool row2_ok(const FourStep &G) { return G.mode == ROW_CONV && G.c >= 9 && G.c <= 13; }
+// Whether the fixed-shape row pass takes this geometry (rows of 2^9 .. 2^13
+// words).
+bool row2_ok(const FourStep &G) { return G.c >= 9 && G.c <= 13; }
+
+template <int CLG>
+static cudaError_t launch_row2_k(const Primes3 &P3, const FourStep &G, const FSJobs &jobs, uint32_t njobs,
+                                 cudaStream_t st) {
+    switch (G.mode) {
+    case ROW_FWD: return launch_row2_t<CLG, RK_FORWARD>(P3, G, jobs, njobs, st);
+    case ROW_ACC_INV: return launch_row2_t<CLG, RK_PIECE>(P3, G, jobs, njobs, st);
+    default:
+        return G.square ? launch_row2_t<CLG, RK_SQUARE>(P3, G, jobs, njobs, st)
+                        : launch_row2_t<CLG, RK_PRODUCT>(P3, G, jobs, njobs, st);
+    }
+}
 
 cudaError_t launch_row2(const Primes3 &P3, const FourStep &G, const FSJobs &jobs, uint32_t njobs, cudaStream_t st) {
-    const bool sq = G.square != 0;
     switch (G.c) {
-    case 9: return sq ? launch_row2_t<9, true>(P3, G, jobs, njobs, st) : launch_row2_t<9, false>(P3, G, jobs, njobs, st);
-    case 10: return sq ? launch_row2_t<10, true>(P3, G, jobs, njobs, st) : launch_row2_t<10, false>(P3, G, jobs, njobs, st);
-    case 11: return sq ? launch_row2_t<11, true>(P3, G, jobs, njobs, st) : launch_row2_t<11, false>(P3, G, jobs, njobs, st);
-    case 12: return sq ? launch_row2_t<12, true>(P3, G, jobs, njobs, st) : launch_row2_t<12, false>(P3, G, jobs, njobs, st);
-    default: return sq ? launch_row2_t<13, true>(P3, G, jobs, njobs, st) : launch_row2_t<13, false>(P3, G, jobs, njobs, st);
+    case 9: return launch_row2_k<9>(P3, G, jobs, njobs, st);
+    case 10: return launch_row2_k<10>(P3, G, jobs, njobs, st);
+    case 11: return launch_row2_k<11>(P3, G, jobs, njobs, st);
+    case 12: return launch_row2_k<12>(P3, G, jobs, njobs, st);
+    default: return launch_row2_k<13>(P3, G, jobs, njobs, st);
     }
 }
 

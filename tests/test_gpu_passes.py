@@ -57,3 +57,23 @@ def test_pass_shapes(ff, rn, c, r3):
             ff.set_geometry(lg, r3, 0, 0)
             ff.load_tuning()
     assert hit
+
+
+@pytest.mark.parametrize("lg", [13, 16, 17, 18, 19, 20])
+def test_split_row_shapes(ff, lg):
+    """The split's row modes at every row length (rows of 2^9 .. 2^13 for
+    pieces of 2^16 .. 2^20 words, and one piece length below): squares with an
+    even and an odd number of pieces, a product of unlike lengths."""
+    ff.init(1 << 20)
+    cap0, max0 = ff.g_ntt_max_L(), ff.ntt_max_L()
+    try:
+        ff.set_max_lg(lg)
+        piece = (1 << lg) // 2 * 32 // 64  # limbs of a piece at width 32
+        for na, nb in ((4 * piece, None), (5 * piece - 7, None), (6 * piece + 3, 2 * piece + 1)):
+            pl = ff.plan(64 * na, 64 * (nb or na), nb is None)
+            assert pl["split"]
+            _check(ff, na, nb or na, nb is None)
+    finally:
+        ff.set_max_lg(25)
+        ff.lib().ffg_set_ntt_max_L(max0)
+        ff.set_g_ntt_max_L(cap0)
