@@ -477,7 +477,7 @@ int run_batch(std::vector<BJob> &jobs, cudaStream_t st, cudaGraph_t *capture) {
         if (ln.key.kernel == 0) {
             ConvJobs cjs{};
             cjs.ext = (const ConvJob *)(dimg + ln.conv_off);
-            e = launch_conv_small(g.P3, cjs, (uint32_t)ln.count, (uint32_t)ln.pl.L, !sq, ls, ln.conv_bytes);
+            e = launch_conv_small(g.P3, cjs, (uint32_t)ln.count, ln.pl.lg, ln.pl.r3, sq, ls, ln.conv_bytes);
             if (e) return end_capture(fail(FFG_E_CUDA, "batched one-CTA transforms: %s", cudaGetErrorString(e)));
         } else {
             FourStep G = four_step_geometry(ln.pl, sq);

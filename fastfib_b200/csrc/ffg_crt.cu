@@ -599,7 +599,10 @@ static bool g_crt_configured = false;
 
 cudaError_t crt_kernel_load() {
     if (g_crt_configured) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_crt<CS_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, k_crt<CS_T>);
+    if (!e) e = cudaFuncGetAttributes(&fa, k_crt<CS_BIG>);
+    if (!e) e = cudaFuncSetAttribute(k_crt<CS_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
     if (!e) e = cudaFuncSetAttribute(k_crt<CS_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_BIG, 1));
     if (!e) e = cudaFuncSetAttribute(k_crt_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
     if (!e) e = cudaFuncSetAttribute(k_crt_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)crt_smem());

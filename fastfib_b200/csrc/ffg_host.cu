@@ -278,6 +278,7 @@ static int build_tables() {
     CK(set_line_consts(lc));
     CK(set_line_consts_rows(lc));
     CK(set_line_consts_cols(lc));
+    CK(set_line_consts_conv(lc));
     return FFG_OK;
 }
 
@@ -536,7 +537,7 @@ static int run_products(const Prod *pr, int count, const ffg_plan &pl, bool squa
             memcpy(J.scls, scls, sizeof scls);
             bytes += 8.0 * (double)(J.na + (square ? 0 : J.nb)) + 12.0 * (double)J.conv;
         }
-        e = launch_conv_small(g.P3, jobs, (uint32_t)count, (uint32_t)L, !square, st, bytes);
+        e = launch_conv_small(g.P3, jobs, (uint32_t)count, pl.lg, pl.r3, square, st, bytes);
         if (e) return fail(FFG_E_CUDA, "conv_small: %s", cudaGetErrorString(e));
     } else {
         FourStep G = four_step_geometry(pl, square);
@@ -1061,6 +1062,7 @@ copy_back:
 using namespace ffg;
 
 static int noalloc_address(int dev, void **addr);
+static int noalloc_kernels_load();
 
 extern "C" int ffg_init(size_t max_limbs) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
@@ -1073,8 +1075,7 @@ extern "C" int ffg_init(size_t max_limbs) {
     CK(cudaGetDevice(&dev));
     void *scratch = nullptr;
     if ((rc = noalloc_address(dev, &scratch))) return rc;
-    CK(ntt_kernels_load()); // and the kernels it launches, for the same reason
-    CK(crt_kernel_load());
+    if ((rc = noalloc_kernels_load())) return rc; // and the kernels it launches, for the same reason
     size_t L = 16;
     while (L < 2 * max_limbs && L < ((size_t)1 << kMaxLg)) L <<= 1;
     if (L > g.max_L) g.max_L = L;
@@ -1352,6 +1353,24 @@ static int noalloc_address(int dev, void **addr) {
     return FFG_OK;
 }
 
+// The kernels that products within that scratch launch at the geometries in
+// force (lengths up to 2^19), once.
+static int noalloc_kernels_load() {
+    static bool done = false;
+    if (done) return FFG_OK;
+    CK(crt_kernel_load());
+    for (uint32_t r3 = 0; r3 < 2; r3++)
+        for (uint32_t lg = 4; lg <= (r3 ? 17u : 19u); lg++) {
+            ffg_plan pl{};
+            pl.lg = lg, pl.r3 = r3, pl.L = (uint64_t)(r3 ? 3 : 1) << lg;
+            gpu_geometry(&pl);
+            for (int square = 0; square < 2; square++)
+                CK(pl.kernel ? load_four_step(four_step_geometry(pl, square != 0)) : load_conv(lg, r3, square != 0));
+        }
+    done = true;
+    return FFG_OK;
+}
+
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 extern "C" int ffg_mul_device_noalloc(uint64_t *out, const uint64_t *a, size_t na, uint64_t bits_a,
@@ -1402,7 +1421,7 @@ extern "C" int ffg_mul_device_noalloc(uint64_t *out, const uint64_t *a, size_t n
         J.n = pl.lg, J.r3 = pl.r3, J.width = w, J.square = square != 0;
         J.conv = (uint32_t)(ca + cb - 1);
         scale_consts(L, J.scl, J.scls);
-        e = launch_conv_small(g.P3, jobs, 1, (uint32_t)L, !square, st,
+        e = launch_conv_small(g.P3, jobs, 1, pl.lg, pl.r3, square != 0, st,
                               8.0 * (double)(na + (square ? 0 : nb)) + 12.0 * (double)J.conv);
     } else {
         FourStep G = four_step_geometry(pl, square != 0);

@@ -240,10 +240,19 @@ bool row2_ok(const FourStep &G);
 cudaError_t launch_row2(const Primes3 &P3, const FourStep &G, const FSJobs &jobs, uint32_t njobs, cudaStream_t st);
 // Load (and configure) the kernels of one product -- the transforms and the
 // plain CRT -- during set-up, so a later first launch loads no module code.
-cudaError_t ntt_kernels_load();
+cudaError_t load_conv(uint32_t n, uint32_t r3, bool square); // one length of the one-CTA convolution
+cudaError_t load_four_step(const FourStep &G);               // one geometry's passes
 cudaError_t crt_kernel_load();
-cudaError_t launch_conv_small(const Primes3 &P3, const ConvJobs &jobs, uint32_t njobs, uint32_t maxL,
-                              bool any_distinct, cudaStream_t st, double bytes);
+cudaError_t launch_conv_small(const Primes3 &P3, const ConvJobs &jobs, uint32_t njobs, uint32_t n, uint32_t r3,
+                              bool square, cudaStream_t st, double bytes);
+// The fixed-length one-CTA convolution (ffg_conv.cu) for the lengths conv2_ok accepts.
+bool conv2_ok(uint32_t n, uint32_t r3);
+cudaError_t launch_conv2(const Primes3 &P3, const ConvJobs &jobs, uint32_t njobs, uint32_t n, uint32_t r3, bool square,
+                         cudaStream_t st);
+cudaError_t load_conv2(uint32_t n, uint32_t r3, bool square);
+cudaError_t load_col2(const FourStep &G);
+cudaError_t load_row2(const FourStep &G);
+cudaError_t set_line_consts_conv(const LineConsts &h); // and ffg_conv.cu
 cudaError_t launch_four_step(const Primes3 &P3, const FourStep &G, const FSJobs &jobs, uint32_t njobs,
                              cudaStream_t st, double limb_bytes);
 cudaError_t launch_split_forward(const Primes3 &P3, FourStep G, const FSJobs &jobs, uint32_t njobs,

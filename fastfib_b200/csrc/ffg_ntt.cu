@@ -3,7 +3,7 @@
 //
 // Short lengths (L <= 2^FFG_LINE_LG words) run one CTA per (product, prime)
 // with the whole transform in shared memory: load digits, forward, pointwise,
-// inverse, scale (k_conv_small).  This is the reference's in-cache
+// inverse, scale (k_conv2, ffg_conv.cu; below 64 words k_conv_small).  This is the reference's in-cache
 // convolution (src/ntt_conv.c:205-226, src/ntt_kernels.c:274-295) as one
 // kernel, and the batched path of the decimal conversion and uneven streams.
 //
@@ -256,21 +256,26 @@ static cudaError_t smem_optin() {
     return cudaSuccess;
 }
 
-cudaError_t ntt_kernels_load() { return smem_optin(); }
-
 static size_t small_smem_bytes(uint32_t L, bool square) {
     return (size_t)line_stride(L) * (square ? 1 : 2) * sizeof(uint32_t);
 }
 
-cudaError_t launch_conv_small(const Primes3 &P3, const ConvJobs &jobs, uint32_t njobs, uint32_t maxL,
-                              bool any_distinct, cudaStream_t st, double bytes) {
-    size_t sm = small_smem_bytes(maxL, !any_distinct);
+// njobs one-CTA convolutions of length 2^n or 3 2^n, all squares or all products:
+// the fixed-length kernel (ffg_conv.cu) where there is one, the generic one for
+// lengths below 64 (and 48, 96).
+cudaError_t launch_conv_small(const Primes3 &P3, const ConvJobs &jobs, uint32_t njobs, uint32_t n, uint32_t r3,
+                              bool square, cudaStream_t st, double bytes) {
     cudaError_t e = smem_optin();
     if (e != cudaSuccess) return e;
     prof_begin(PK_CONV_SMALL, st);
-    k_conv_small<<<dim3(njobs, 3, 1), 256, sm, st>>>(P3, jobs);
+    if (conv2_ok(n, r3)) {
+        e = launch_conv2(P3, jobs, njobs, n, r3, square, st);
+    } else {
+        k_conv_small<<<dim3(njobs, 3, 1), 256, small_smem_bytes((r3 ? 3u : 1u) << n, square), st>>>(P3, jobs);
+        e = cudaGetLastError();
+    }
     prof_end(PK_CONV_SMALL, st, bytes);
-    return cudaGetLastError();
+    return e;
 }
 
 // The fixed-shape row pass (ffg_rows.cu) where it applies; FFG_ROW2=0 keeps
@@ -334,6 +339,18 @@ cudaError_t launch_four_step(const Primes3 &P3, const FourStep &G, const FSJobs 
         e = cudaGetLastError();
     }
     prof_end(PK_COL_INV, st, res * 2);
+    return e;
+}
+
+cudaError_t load_conv(uint32_t n, uint32_t r3, bool square) {
+    cudaError_t e = smem_optin();
+    return e || !conv2_ok(n, r3) ? e : load_conv2(n, r3, square);
+}
+
+cudaError_t load_four_step(const FourStep &G) {
+    cudaError_t e = smem_optin();
+    if (!e && g_col2 && col2_ok(G)) e = load_col2(G);
+    if (!e && g_row2 && row2_ok(G)) e = load_row2(G);
     return e;
 }
 

@@ -31,6 +31,8 @@
 // It computes the same residues as the generic row pass of ffg_ntt.cu
 // (k_row_conv): the order of the frequencies between the forward and the
 // inverse differs, but the pointwise product does not care.
+#include <utility>
+
 #include "ffg_internal.h"
 #include "ffg_lines.cuh"
 
@@ -277,18 +279,26 @@ __global__ void __launch_bounds__(256, CLG == 13 && KIND == RK_PRODUCT ? 3 : 4) 
     }
 }
 
+// Loads a kernel and opts it into its shared memory, once.
+template <int CLG, int KIND> static cudaError_t load_row2_t() {
+    using Q = RowGeo<CLG>;
+    static bool attr = false;
+    if (attr) return cudaSuccess;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, k_row2<CLG, KIND>);
+    const size_t smax = (size_t)Q::ROWS * (KIND == RK_PRODUCT ? 2 : 1) * Q::LS * sizeof(uint32_t);
+    if (!e) e = cudaFuncSetAttribute(k_row2<CLG, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
+    if (!e) attr = true;
+    return e;
+}
+
 template <int CLG, int KIND>
 static cudaError_t launch_row2_t(const Primes3 &P3, const FourStep &G, const FSJobs &jobs, uint32_t njobs,
                                  cudaStream_t st) {
     using Q = RowGeo<CLG>;
     constexpr uint32_t lines = KIND == RK_PRODUCT ? 2 : 1;
-    const size_t smax = (size_t)Q::ROWS * lines * Q::LS * sizeof(uint32_t);
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_row2<CLG, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
-        if (e) return e;
-        attr = true;
-    }
+    cudaError_t e = load_row2_t<CLG, KIND>();
+    if (e) return e;
     // rows per CTA: as many as fit 256 threads, halved while the launch would
     // have fewer than three CTAs per SM (short rows of a mid-size product)
     uint32_t rows = Q::ROWS;
@@ -302,6 +312,17 @@ static cudaError_t launch_row2_t(const Primes3 &P3, const FourStep &G, const FSJ
 // This unit's copy of the line-transform constants (each CUDA unit has its
 // own constant bank); set once with the others.
 cudaError_t set_line_consts_rows(const LineConsts &h) { return cudaMemcpyToSymbol(c_lines, &h, sizeof h); }
+
+template <int... CLG> static cudaError_t load_row2_c(uint32_t c, bool square, std::integer_sequence<int, CLG...>) {
+    cudaError_t e = cudaSuccess;
+    ((c == CLG + 9 ? (void)(e = square ? load_row2_t<CLG + 9, RK_SQUARE>() : load_row2_t<CLG + 9, RK_PRODUCT>())
+                   : (void)0),
+     ...);
+    return e;
+}
+cudaError_t load_row2(const FourStep &G) {
+    return load_row2_c(G.c, G.square != 0, std::make_integer_sequence<int, 5>{}); // 2^9 .. 2^13
+}
 
 // Whether the fixed-shape row pass takes this geometry (rows of 2^9 .. 2^13
 // words).

@@ -77,3 +77,36 @@ def test_split_row_shapes(ff, lg):
         ff.set_max_lg(25)
         ff.lib().ffg_set_ntt_max_L(max0)
         ff.set_g_ntt_max_L(cap0)
+
+
+def test_one_cta_lengths(ff):
+    """The one-CTA convolution at every length 2^4 .. 2^14 and 3 2^4 .. 3 2^12:
+    batches of 64 products (which run it past 4096 words too) with operands
+    around half of the length, a short one, nearly full ones, for products and
+    squares, against Python integers."""
+    ff.init(1 << 20)
+    rng = np.random.default_rng(3)
+    lengths = set()
+    for r3, top in ((0, 14), (1, 12)):
+        for lg in range(4, top + 1):
+            L = (3 if r3 else 1) << lg
+            for na, nb in ((L // 4, None), (max(1, L // 4 - 1), L // 4), (max(1, L // 2 - L // 16 - 1), max(1, L // 32)),
+                           (L // 4 + max(1, L // 128), None)):
+                pl = ff.plan(64 * na, 64 * (nb or na), nb is None)
+                if pl["L"] != L or pl["split"]:
+                    continue
+                pairs = []
+                for _ in range(64):
+                    a = rng.integers(0, 2**64, na, dtype=np.uint64)
+                    a[-1] |= np.uint64(1 << 63)
+                    b = None
+                    if nb:
+                        b = rng.integers(0, 2**64, nb, dtype=np.uint64)
+                        b[-1] |= np.uint64(1 << 63)
+                    pairs.append((a, b))
+                lengths.add(L)
+                for (a, b), out in zip(pairs[:6], ff.mul_batch(pairs, method="ntt")[:6]):
+                    x = ff.limbs_to_int(a)
+                    y = x if b is None else ff.limbs_to_int(b)
+                    assert ff.limbs_to_int(out) == x * y, (L, na, nb)
+    assert len(lengths) >= 18
