@@ -177,9 +177,19 @@ uint32_t crt_ctas(uint64_t nlimbs, uint32_t width) {
 
 constexpr int CS_T = CRT_COEF / 32;  // super-limbs of a CTA (64), the unit of crt_ctas()
 constexpr int CS_BIG = 256;          // super-limbs of a CTA of a long product
-constexpr uint32_t CS_ROW = 36;      // shared words of a row (32 coefficients' words; the b words of output)
-// shared words of one word of every value of T super-limbs
-template <int T> __host__ __device__ constexpr uint32_t cs_plane() { return T * CS_ROW; }
+// T super-limbs of SL coefficients of width B: W words of output each; shared
+// words of a row (SL coefficients' words, later the W words of output; rows 4
+// words apart from a power of two keep 16-byte accesses off each other's banks)
+// and of a plane (one word of every value).
+template <int T, int SL, int B> struct CrtGeo {
+    static constexpr int W = SL * B / 32;
+    static constexpr uint32_t ROW = SL + 4, PLANE = T * ROW;
+    static_assert(SL * B % 32 == 0 && W <= (int)ROW && W >= 8 && SL >= 8 && T % 32 == 0, "whole words");
+};
+// The shortest super-limbs of a width (short products: the sums' serial chain).
+template <int B> struct CrtShort {
+    static constexpr int SL = B == 32 ? 8 : (B == 34 ? 16 : 32);
+};
 
 // Garner's X as words x[0] + 2^32 x[1] + 2^64 x[2].
 FFG_DEV_INLINE u128 garner_lean(const GarnerConst &K, uint32_t r1, uint32_t r2, uint32_t r3) {
@@ -220,7 +230,8 @@ struct Super {
 // loaded before chunk c's words are stored; b words for 32 never overtake it).
 // eval(a, b, c): the value of a coefficient from its words in the three planes
 // (a value's own words, or residues not yet recombined).
-template <int T, int B, class Eval> FFG_DEV_INLINE void super_sum(Super &S, uint32_t *row, bool all, Eval value) {
+template <class Q, int SL, int B, class Eval>
+FFG_DEV_INLINE void super_sum(Super &S, uint32_t *row, bool all, Eval value) {
     u128 acc = 0, last[4];
     uint32_t w[4], buf[4];
     S.ones = ~0u;
@@ -229,7 +240,7 @@ template <int T, int B, class Eval> FFG_DEV_INLINE void super_sum(Super &S, uint
     } cur, nxt;
     auto load = [&](int c, Raw &q) {
 #pragma unroll
-        for (int k = 0; k < 3; k++) q.r[k] = *(const uint4 *)(row + k * cs_plane<T>() + 4 * c);
+        for (int k = 0; k < 3; k++) q.r[k] = *(const uint4 *)(row + k * Q::PLANE + 4 * c);
     };
     auto eval = [&](const Raw &q, int e) { return value(quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e)); };
     load(0, cur);
@@ -259,9 +270,9 @@ template <int T, int B, class Eval> FFG_DEV_INLINE void super_sum(Super &S, uint
     chunk(0, cur);
     if (B == 32) {
 #pragma unroll 1
-        for (int c = 1; c < 8; c++) {
+        for (int c = 1; c < SL / 4; c++) {
             cur = nxt;
-            if (c < 7) load(c + 1, nxt);
+            if (c + 1 < SL / 4) load(c + 1, nxt);
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 last[e] = eval(cur, e);
@@ -274,13 +285,13 @@ template <int T, int B, class Eval> FFG_DEV_INLINE void super_sum(Super &S, uint
         }
     } else {
 #pragma unroll
-        for (int c = 1; c < 8; c++) {
+        for (int c = 1; c < SL / 4; c++) {
             cur = nxt;
-            if (c < 7) load(c + 1, nxt);
+            if (c + 1 < SL / 4) load(c + 1, nxt);
             chunk(c, cur);
         }
 #pragma unroll
-        for (int m = 0; m < B % 4; m++) row[(B & ~3) + m] = buf[m];
+        for (int m = 0; m < Q::W % 4; m++) row[(Q::W & ~3) + m] = buf[m];
     }
     S.w01 = (uint64_t)w[1] << 32 | w[0];
     S.w23 = (uint64_t)w[3] << 32 | w[2];
@@ -290,12 +301,12 @@ template <int T, int B, class Eval> FFG_DEV_INLINE void super_sum(Super &S, uint
 
 FFG_DEV_INLINE u128 words_value(uint32_t a, uint32_t b, uint32_t c) { return (u128)c << 64 | (uint64_t)b << 32 | a; }
 
-// Adds v to words 4 .. b - 1 (v = 1 or -1, a carry or a borrow out of the words
+// Adds v to words 4 .. W - 1 (v = 1 or -1, a carry or a borrow out of the words
 // below): rare.  Returns the carry or borrow out of the super-limb.
-template <int B> FFG_DEV_INLINE bool super_ripple(Super &S, uint32_t *row, uint32_t v) {
+template <int W> FFG_DEV_INLINE bool super_ripple(Super &S, uint32_t *row, uint32_t v) {
     bool on = true;
     uint32_t ones = ~0u;
-    for (int k = 4; k < B; k++) {
+    for (int k = 4; k < W; k++) {
         uint32_t x = row[k];
         if (on) {
             on = v == 1 ? x == ~0u : x == 0;
@@ -321,7 +332,7 @@ struct SuperShared {
 // (the others' is their neighbour's left).  sub > 0: the constant is -sub in the
 // first limb's super-limb (1 in the others), in two's complement over the whole
 // number.
-template <int T, int B>
+template <int T, int W>
 FFG_DEV_INLINE uint32_t super_resolve(Super &S, uint32_t *row, SuperShared &sh, uint64_t cin, uint64_t sub) {
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr uint32_t NW = T / 32;
@@ -333,7 +344,7 @@ FFG_DEV_INLINE uint32_t super_resolve(Super &S, uint32_t *row, SuperShared &sh, 
             if (br) {
                 br = S.w23 == 0;
                 S.w23 -= 1;
-                if (br) br = super_ripple<B>(S, row, ~0u);
+                if (br) br = super_ripple<W>(S, row, ~0u);
             }
             S.left += !br;
         }
@@ -348,7 +359,7 @@ FFG_DEV_INLINE uint32_t super_resolve(Super &S, uint32_t *row, SuperShared &sh, 
         S.w01 += h;
         if (S.w01 < h) {
             S.w23 += 1;
-            if (S.w23 == 0) G = super_ripple<B>(S, row, 1);
+            if (S.w23 == 0) G = super_ripple<W>(S, row, 1);
         }
         const bool P = !G && (S.w01 & S.w23) == ~0ull && S.ones == ~0u;
         Gm = __ballot_sync(0xffffffffu, G), Pm = __ballot_sync(0xffffffffu, P);
@@ -369,7 +380,7 @@ FFG_DEV_INLINE uint32_t super_resolve(Super &S, uint32_t *row, SuperShared &sh, 
         }
         const uint64_t A = Gm | Pm, Bm = Gm;
         if ((((uint32_t)((A + Bm + cw) ^ A ^ Bm)) >> lane) & 1u) {
-            if (++S.w01 == 0 && ++S.w23 == 0) super_ripple<B>(S, row, 1);
+            if (++S.w01 == 0 && ++S.w23 == 0) super_ripple<W>(S, row, 1);
         }
         *(uint4 *)row = make_uint4((uint32_t)S.w01, (uint32_t)(S.w01 >> 32), (uint32_t)S.w23, (uint32_t)(S.w23 >> 32));
     }
@@ -379,18 +390,19 @@ FFG_DEV_INLINE uint32_t super_resolve(Super &S, uint32_t *row, SuperShared &sh, 
     return (d + c0) | ((d + c1) << 1);
 }
 
-// The CTA's words (rows of b) to its T b / 2 limbs from j0 of out, below nlimbs.
-template <int T, int B> FFG_DEV_INLINE void super_store(const uint32_t *rows, uint64_t *out, uint64_t j0, uint64_t nlimbs) {
-    const uint32_t nl = T * B / 2;
+// The CTA's words (rows of W) to its T W / 2 limbs from j0 of out, below nlimbs.
+template <int T, int W, uint32_t ROW>
+FFG_DEV_INLINE void super_store(const uint32_t *rows, uint64_t *out, uint64_t j0, uint64_t nlimbs) {
+    const uint32_t nl = T * W / 2;
     const uint32_t lim = nlimbs > j0 ? (nlimbs - j0 < nl ? (uint32_t)(nlimbs - j0) : nl) : 0;
     for (uint32_t l = threadIdx.x; l < lim; l += blockDim.x) {
-        const uint32_t k = 2 * l, r = k / B, c = k - r * B;
+        const uint32_t k = 2 * l, r = k / W, c = k - r * W;
         uint64_t v;
-        if (B % 2 == 0) {
-            v = *(const uint64_t *)(rows + r * CS_ROW + c);
+        if (W % 2 == 0) {
+            v = *(const uint64_t *)(rows + r * ROW + c);
         } else {
-            const uint32_t lo = rows[r * CS_ROW + c];
-            const uint32_t hi = c + 1 < B ? rows[r * CS_ROW + c + 1] : rows[(r + 1) * CS_ROW];
+            const uint32_t lo = rows[r * ROW + c];
+            const uint32_t hi = c + 1 < W ? rows[r * ROW + c + 1] : rows[(r + 1) * ROW];
             v = (uint64_t)hi << 32 | lo;
         }
         out[j0 + l] = v;
@@ -410,7 +422,7 @@ FFG_DEV_INLINE void halo_value(const uint32_t (&h)[3][4], u128 (&x)[4]) {
 // Residues of the CTA's coefficients (and of the 4 below it) into three planes,
 // zero at or past conv (Garner of zeros is zero): cp.async, so that a CTA's loads
 // are all in flight at once without a register each.
-template <int T>
+template <int NT, class Q, int T, int SL>
 FFG_DEV_INLINE void super_stage(uint32_t *planes, uint32_t (&halo)[3][4], const uint32_t *y, uint64_t stride,
                                 int64_t ibase, uint64_t conv) {
     auto copy = [&](uint32_t *dst, const uint32_t *src, int64_t gi) {
@@ -422,11 +434,11 @@ FFG_DEV_INLINE void super_stage(uint32_t *planes, uint32_t (&halo)[3][4], const 
 #pragma unroll
     for (int k = 0; k < 3; k++) {
 #pragma unroll
-        for (uint32_t v = 0; v < 8; v++) {
-            const uint32_t q = threadIdx.x + v * T;
-            copy(planes + k * cs_plane<T>() + (q >> 3) * CS_ROW + (q & 7) * 4, y + k * stride, ibase + 4 * (int64_t)q);
+        for (uint32_t v = 0; v < T * SL / 4 / NT; v++) {
+            const uint32_t q = threadIdx.x + v * NT;
+            copy(planes + k * Q::PLANE + q / (SL / 4) * Q::ROW + q % (SL / 4) * 4, y + k * stride, ibase + 4 * (int64_t)q);
         }
-        if (threadIdx.x == T - 1) copy(halo[k], y + k * stride, ibase - 4);
+        if (threadIdx.x == NT - 1) copy(halo[k], y + k * stride, ibase - 4);
     }
 }
 FFG_DEV_INLINE void super_staged() {
@@ -438,7 +450,7 @@ FFG_DEV_INLINE void super_staged() {
 // of coefficients gi .. gi + 3, eval(raw, e, z) gives the values of the e-th.
 // A thread's loads are issued before any arithmetic; lanes 0..3 of the last
 // warp also do one coefficient each of the 4 below the CTA.
-template <int NT, int NO, class Raw, class Ld, class Eval>
+template <int NT, class Q, int SL, int NO, class Raw, class Ld, class Eval>
 FFG_DEV_INLINE void super_fill(uint32_t *planes, CrtShared &sh, int64_t ibase, Ld ld, Eval eval) {
     constexpr uint32_t PER = CRT_COEF / 4 / NT, AHEAD = NO == 1 ? 2 : 1; // quads a thread, AHEAD loaded at a time
     const uint32_t t = threadIdx.x, low = t - (NT - 32); // 0..3: a coefficient below the CTA
@@ -455,12 +467,12 @@ FFG_DEV_INLINE void super_fill(uint32_t *planes, CrtShared &sh, int64_t ibase, L
 #pragma unroll
                 for (int m = 0; m < 3; m++) x[k][m][e] = (uint32_t)(z[k] >> (32 * m));
         }
-        uint32_t *d = planes + (q >> 3) * CS_ROW + (q & 7) * 4;
+        uint32_t *d = planes + q / (SL / 4) * Q::ROW + q % (SL / 4) * 4;
 #pragma unroll
         for (int k = 0; k < NO; k++)
 #pragma unroll
             for (int m = 0; m < 3; m++)
-                *(uint4 *)(d + (3 * k + m) * cs_plane<CS_T>()) =
+                *(uint4 *)(d + (3 * k + m) * Q::PLANE) =
                     make_uint4(x[k][m][0], x[k][m][1], x[k][m][2], x[k][m][3]);
     };
 #pragma unroll 1
@@ -501,65 +513,83 @@ FFG_DEV_INLINE void ld_residues(uint4 *r, const uint32_t *y, uint64_t stride, in
     }
 }
 
-// T = CS_T: Garner by all NT threads, sums by T of them (short products: a
-// thread recombines 8 coefficients and adds 32; batches).  T = CS_BIG = NT: every
-// thread recombines and adds its own 32 coefficients in one pass with no barrier
-// in between, and there are a quarter of the carry maps; the latency of 32
-// coefficients a thread does not count when the CTAs fill the GPU twice over.
-template <int NT, int T, int B>
+// How a CTA runs a CRT.
+enum CrtForm {
+    // short products: 256 threads recombine two quads each from registers, the
+    // sums run over short super-limbs (the time is one thread's chain)
+    CF_SHORT,
+    // batches of products of any size: the same with 128 threads and super-limbs
+    // of 32
+    CF_BATCH,
+    // CTAs of 256 super-limbs: every thread recombines and adds its own 32
+    // coefficients in one pass with no barrier in between, and there are a quarter
+    // of the carry maps; for launches that fill the GPU twice over
+    CF_LONG
+};
+template <CrtForm F> __host__ __device__ constexpr int crt_threads() { return F == CF_BATCH ? 128 : 256; }
+
+template <CrtForm F, int B>
 FFG_DEV_INLINE void crt_super(const GarnerConst &K, const CrtJob &J, uint32_t cta, uint32_t *planes, CrtShared &sh) {
+    constexpr int NT = crt_threads<F>(), SL = F == CF_SHORT ? CrtShort<B>::SL : 32;
+    constexpr int T = F == CF_LONG ? CS_BIG : CRT_COEF / SL;
+    using Q = CrtGeo<T, SL, B>;
+    constexpr uint32_t NL = T * Q::W / 2; // limbs
     const uint32_t t = threadIdx.x;
-    const int64_t ibase = (int64_t)cta * (32 * T);
-    uint32_t *const row = planes + t * CS_ROW;
+    const int64_t ibase = (int64_t)cta * (SL * T);
+    uint32_t *const row = planes + t * Q::ROW;
     const bool neg = J.add < 0;
     Super S;
     uint64_t cin = 0;
     u128 below[4];
     auto garner = [&](uint32_t a, uint32_t b, uint32_t c) { return garner_lean(K, a, b, c); };
-    if (NT == T) {
-        super_stage<T>(planes, sh.halo[0], J.y, J.y_stride, ibase, J.conv);
+    if (F != CF_LONG) {
+        super_fill<NT, Q, SL, 1, Raw3>(
+            planes, sh, ibase, [&](int64_t gi, Raw3 &q) { ld_residues(q.r, J.y, J.y_stride, gi, J.conv); },
+            [&](const Raw3 &q, int e, u128(&x)[1]) {
+                x[0] = garner(quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e));
+            });
+    } else {
+        super_stage<NT, Q, T, SL>(planes, sh.halo[0], J.y, J.y_stride, ibase, J.conv);
         super_staged();
-        super_sum<T, B>(S, row, neg, garner);
+    }
+    if (F == CF_LONG) {
+        super_sum<Q, SL, B>(S, row, neg, garner);
         if (t == 0) {
 #pragma unroll
             for (int e = 0; e < 4; e++) below[e] = garner(sh.halo[0][0][e], sh.halo[0][1][e], sh.halo[0][2][e]);
         }
     } else {
-        super_fill<NT, 1, Raw3>(
-            planes, sh, ibase, [&](int64_t gi, Raw3 &q) { ld_residues(q.r, J.y, J.y_stride, gi, J.conv); },
-            [&](const Raw3 &q, int e, u128(&x)[1]) {
-                x[0] = garner(quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e));
-            });
-        if (t < T) super_sum<T, B>(S, row, neg, words_value);
+        if (t < T) super_sum<Q, SL, B>(S, row, neg, words_value);
         if (t == 0) halo_value(sh.halo[0], below);
     }
     if (t == 0) cin = cta ? boundary_carry<B>(below, neg) : (neg ? 0 : (uint64_t)J.add);
     const uint64_t sub = neg ? (t == 0 && cta == 0 ? (uint64_t)-J.add : 1) : 0;
-    const uint32_t map = super_resolve<T, B>(S, row, sh.sup, cin, sub);
-    super_store<T, B>(planes, J.out, (uint64_t)cta * (T * B / 2), J.nlimbs);
-    const uint32_t ncta = (uint32_t)((J.nlimbs + T * B / 2 - 1) / (T * B / 2));
+    const uint32_t map = super_resolve<T, Q::W>(S, row, sh.sup, cin, sub);
+    super_store<T, Q::W, Q::ROW>(planes, J.out, (uint64_t)cta * NL, J.nlimbs);
+    const uint32_t ncta = (uint32_t)((J.nlimbs + NL - 1) / NL);
     if (ncta > 1) {
         if (t == 0) J.maps[cta] = map;
         if (last_cta(J.ticket, ncta)) {
-            settle_cta(J.out, J.nlimbs, T * B / 2, J.maps, ncta);
+            settle_cta(J.out, J.nlimbs, NL, J.maps, ncta);
             if (t == 0) *J.ticket = 0;
         }
     }
 }
 
-template <int NT, int T> FFG_DEV_INLINE void crt_any(const GarnerConst &K, const CrtJob &J, uint32_t cta) {
+template <CrtForm F> FFG_DEV_INLINE void crt_any(const GarnerConst &K, const CrtJob &J, uint32_t cta) {
     extern __shared__ __align__(16) uint32_t cs_rows[];
     __shared__ CrtShared sh;
     switch (J.width) {
-    case 32: crt_super<NT, T, 32>(K, J, cta, cs_rows, sh); return;
-    case 33: crt_super<NT, T, 33>(K, J, cta, cs_rows, sh); return;
-    case 34: crt_super<NT, T, 34>(K, J, cta, cs_rows, sh); return;
-    default: crt_super<NT, T, 35>(K, J, cta, cs_rows, sh); return;
+    case 32: crt_super<F, 32>(K, J, cta, cs_rows, sh); return;
+    case 33: crt_super<F, 33>(K, J, cta, cs_rows, sh); return;
+    case 34: crt_super<F, 34>(K, J, cta, cs_rows, sh); return;
+    default: crt_super<F, 35>(K, J, cta, cs_rows, sh); return;
     }
 }
 
-template <int T> __global__ void __launch_bounds__(256, T == CS_BIG ? 2 : 3) k_crt(GarnerConst K, CrtJob J) {
-    crt_any<256, T>(K, J, blockIdx.x);
+template <CrtForm F>
+__global__ void __launch_bounds__(crt_threads<F>(), F == CF_BATCH ? 6 : (F == CF_SHORT ? 3 : 2)) k_crt(GarnerConst K, CrtJob J) {
+    crt_any<F>(K, J, blockIdx.x);
 }
 
 // Up to two CRTs by value (the doubling step's two squarings): product
@@ -570,7 +600,7 @@ struct CrtPair {
 __global__ void __launch_bounds__(256, 3) k_crt_pair(GarnerConst K, CrtPair P) {
     const CrtJob J = blockIdx.y ? P.j[1] : P.j[0];
     if (blockIdx.x >= crt_ctas_dev(J.nlimbs, J.width)) return;
-    crt_any<256, CS_T>(K, J, blockIdx.x);
+    crt_any<CF_SHORT>(K, J, blockIdx.x);
 }
 
 // CRTs of any sizes in one launch: CTA b runs CTA b - first[j] of job j,
@@ -586,10 +616,16 @@ __global__ void __launch_bounds__(128, 6) k_crt_flat(GarnerConst K, const CrtJob
         else hi = mid;
     }
     const CrtJob J = jobs[lo];
-    crt_any<128, CS_T>(K, J, b - __ldg(&first[lo]));
+    crt_any<CF_BATCH>(K, J, b - __ldg(&first[lo]));
 }
 
-static size_t super_smem(uint32_t T, uint32_t outs) { return (size_t)3 * outs * T * CS_ROW * sizeof(uint32_t); }
+// Shared bytes of T super-limbs' planes (the widest rows: SL + 4 words for 8
+// coefficients and more) of n values.
+template <int T, int SL> constexpr size_t super_smem(uint32_t n) {
+    return (size_t)3 * n * T * (SL + 4) * sizeof(uint32_t);
+}
+constexpr size_t kShortSmem = super_smem<CRT_COEF / 8, 8>(1), kBatchSmem = super_smem<CS_T, 32>(1),
+                 kLongSmem = super_smem<CS_BIG, 32>(1);
 
 static size_t crt_smem() {
     return (CRT_COEF + CRT_HALO_MAX) * (8 + 4) + CRT_NL_MAX * (8 + 4) + 3 * (CRT_NL_MAX / 32) * 4;
@@ -600,11 +636,11 @@ static bool g_crt_configured = false;
 cudaError_t crt_kernel_load() {
     if (g_crt_configured) return cudaSuccess;
     cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, k_crt<CS_T>);
-    if (!e) e = cudaFuncGetAttributes(&fa, k_crt<CS_BIG>);
-    if (!e) e = cudaFuncSetAttribute(k_crt<CS_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
-    if (!e) e = cudaFuncSetAttribute(k_crt<CS_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_BIG, 1));
-    if (!e) e = cudaFuncSetAttribute(k_crt_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
+    cudaError_t e = cudaFuncGetAttributes(&fa, k_crt<CF_SHORT>);
+    if (!e) e = cudaFuncGetAttributes(&fa, k_crt<CF_LONG>);
+    if (!e) e = cudaFuncSetAttribute(k_crt<CF_SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShortSmem);
+    if (!e) e = cudaFuncSetAttribute(k_crt<CF_LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongSmem);
+    if (!e) e = cudaFuncSetAttribute(k_crt_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShortSmem);
     if (!e) e = cudaFuncSetAttribute(k_crt_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)crt_smem());
     if (e) return e;
     g_crt_configured = true;
@@ -615,6 +651,8 @@ cudaError_t crt_kernel_load() {
 // (at 2^22 coefficients, 2049 against 513 CTAs, 32.0 against 25.1 us; below,
 // CTAs of 256 leave SMs idle).
 constexpr uint32_t kCrtBigCtas = 1024;
+// Up to this many CTAs (two an SM) a product runs the short form.
+constexpr uint32_t kCrtShortCtas = 296;
 
 cudaError_t launch_crt(const Primes3 &P3, const CrtJob &J, cudaStream_t st) {
     (void)P3;
@@ -623,8 +661,9 @@ cudaError_t launch_crt(const Primes3 &P3, const CrtJob &J, cudaStream_t st) {
     const uint32_t ncta = crt_ctas(J.nlimbs, J.width);
     prof_begin(PK_CRT, st);
     if (J.width < 32) k_crt_narrow<<<ncta, CRT_THREADS, crt_smem(), st>>>(garner_const(), J);
-    else if (ncta <= kCrtBigCtas) k_crt<CS_T><<<ncta, 256, super_smem(CS_T, 1), st>>>(garner_const(), J);
-    else k_crt<CS_BIG><<<(ncta + 3) / 4, 256, super_smem(CS_BIG, 1), st>>>(garner_const(), J);
+    else if (ncta <= kCrtShortCtas) k_crt<CF_SHORT><<<ncta, 256, kShortSmem, st>>>(garner_const(), J);
+    else if (ncta <= kCrtBigCtas) k_crt<CF_BATCH><<<ncta, 128, kBatchSmem, st>>>(garner_const(), J);
+    else k_crt<CF_LONG><<<(ncta + 3) / 4, 256, kLongSmem, st>>>(garner_const(), J);
     prof_end(PK_CRT, st, 12.0 * (double)J.conv + 8.0 * (double)J.nlimbs);
     return cudaGetLastError();
 }
@@ -644,7 +683,7 @@ cudaError_t launch_crt_pair(const CrtJob *jobs, uint32_t count, cudaStream_t st)
     double bytes = 0;
     for (int i = 0; i < 2; i++) bytes += 12.0 * (double)jobs[i].conv + 8.0 * (double)jobs[i].nlimbs;
     prof_begin(PK_CRT, st);
-    k_crt_pair<<<dim3(n0 > n1 ? n0 : n1, 2), 256, super_smem(CS_T, 1), st>>>(garner_const(), P);
+    k_crt_pair<<<dim3(n0 > n1 ? n0 : n1, 2), 256, kShortSmem, st>>>(garner_const(), P);
     prof_end(PK_CRT, st, bytes);
     return cudaGetLastError();
 }
@@ -653,7 +692,7 @@ cudaError_t launch_crt_flat(const CrtJob *d_jobs, const uint32_t *d_first, uint3
                             cudaStream_t st, double bytes) {
     if (!count || !total_ctas) return cudaSuccess;
     prof_begin(PK_CRT, st);
-    k_crt_flat<<<total_ctas, 128, super_smem(CS_T, 1), st>>>(garner_const(), d_jobs, d_first, count);
+    k_crt_flat<<<total_ctas, 128, kBatchSmem, st>>>(garner_const(), d_jobs, d_first, count);
     prof_end(PK_CRT, st, bytes);
     return cudaGetLastError();
 }
@@ -671,13 +710,41 @@ cudaError_t launch_crt_flat(const CrtJob *d_jobs, const uint32_t *d_first, uint3
 // 2^(64 len) that falls off the top (N b >= 64 len).  The rest is crt_super
 // with values of up to 96 bits.  kOuts 1: output blockIdx.y alone (short
 // products, where twice the CTAs hide more than recombining twice costs); 2:
-// both outputs from one recombination.
+// both outputs from one recombination (as CF_BATCH).  kOuts 1: 512 threads stage the
+// residues, recombine a coefficient at a time in a rolled loop (straight-line code
+// for 16 of them would take longer to fetch than to run) and add short super-limbs:
+// 12.5 -> 10.7 us a step of the F(10^8) chain against CF_SHORT's form.
 struct Raw6 {
     uint4 r[6];
 };
 
-template <int NT, int B, int kOuts>
+// Values in place of the staged residues, a coefficient at a time in a rolled loop:
+// value(d, p, h, hp) from the words at d, d + p, d + 2 p and h, h + hp, h + 2 hp of
+// its two squarings.
+template <int NT, class Q, int SL, class Value>
+FFG_DEV_INLINE void short_values(uint32_t *planes, uint32_t (*halo)[3][4], Value value) {
+    auto put = [&](uint32_t *d, uint32_t pitch, uint32_t *h, uint32_t hp) {
+        const u128 z = value(d, pitch, h, hp);
+        d[0] = (uint32_t)z;
+        d[pitch] = (uint32_t)(z >> 32);
+        d[2 * pitch] = (uint32_t)(z >> 64);
+    };
+#pragma unroll 2
+    for (uint32_t v = threadIdx.x; v < CRT_COEF; v += NT) {
+        uint32_t *d = planes + v / SL * Q::ROW + v % SL;
+        put(d, Q::PLANE, d + 3 * Q::PLANE, Q::PLANE);
+    }
+    const uint32_t low = threadIdx.x - (NT - 32); // 0..3: a coefficient below the CTA
+    if (low < 4) put(&halo[0][0][low], 4, &halo[1][0][low], 4);
+    __syncthreads();
+}
+
+template <int kOuts> __host__ __device__ constexpr int crt_lin_threads() { return kOuts == 1 ? 512 : 128; }
+
+template <int B, int kOuts>
 FFG_DEV_INLINE void crt_lin_super(const GarnerConst &K, const CrtLinJob &J, uint32_t *planes, CrtShared &sh) {
+    constexpr int NT = crt_lin_threads<kOuts>(), SL = kOuts == 1 ? CrtShort<B>::SL : 32, T = CRT_COEF / SL;
+    using Q = CrtGeo<T, SL, B>;
     const uint32_t t = threadIdx.x, cta = blockIdx.x, ncta = gridDim.x;
     const int64_t ibase = (int64_t)cta * CRT_COEF;
     const int k0 = kOuts == 1 ? (int)blockIdx.y : 0;
@@ -690,28 +757,39 @@ FFG_DEV_INLINE void crt_lin_super(const GarnerConst &K, const CrtLinJob &J, uint
         al[k] = (uint32_t)(k0 + k ? J.alpha[1] : J.alpha[0]);
         be[k] = k0 + k ? J.beta[1] : J.beta[0];
     }
-    auto eval = [&](const Raw6 &q, int e, u128(&z)[kOuts]) {
-        const u128 x1 = garner_lean(K, quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e));
-        const u128 x2 = garner_lean(K, quad_word(q.r[3], e), quad_word(q.r[4], e), quad_word(q.r[5], e));
-#pragma unroll
-        for (int k = 0; k < kOuts; k++) { // exact mod 2^128, 0 <= z < 2^96
-            const u128 v = x1 * al[k] + bias;
-            z[k] = be[k] >= 0 ? v + x2 * (uint32_t)be[k] : v - x2 * (uint32_t)(-be[k]);
-        }
+    auto combine = [&](u128 x1, u128 x2, int k) { // exact mod 2^128, 0 <= z < 2^96
+        const u128 v = x1 * al[k] + bias;
+        return be[k] >= 0 ? v + x2 * (uint32_t)be[k] : v - x2 * (uint32_t)(-be[k]);
     };
-    super_fill<NT, kOuts, Raw6>(
-        planes, sh, ibase,
-        [&](int64_t gi, Raw6 &q) {
-            ld_residues(q.r, J.y[0], J.y_stride, gi, conv0);
-            ld_residues(q.r + 3, J.y[1], J.y_stride, gi, conv1);
-        },
-        eval);
+    if (kOuts == 1) {
+        super_stage<NT, Q, T, SL>(planes, sh.halo[0], J.y[0], J.y_stride, ibase, conv0);
+        super_stage<NT, Q, T, SL>(planes + 3 * Q::PLANE, sh.halo[1], J.y[1], J.y_stride, ibase, conv1);
+        super_staged();
+        short_values<NT, Q, SL>(planes, sh.halo,
+                                [&](const uint32_t *d, uint32_t p, const uint32_t *h, uint32_t hp) {
+                                    return combine(garner_lean(K, d[0], d[p], d[2 * p]),
+                                                   garner_lean(K, h[0], h[hp], h[2 * hp]), 0);
+                                });
+    } else {
+        super_fill<NT, Q, SL, kOuts, Raw6>(
+            planes, sh, ibase,
+            [&](int64_t gi, Raw6 &q) {
+                ld_residues(q.r, J.y[0], J.y_stride, gi, conv0);
+                ld_residues(q.r + 3, J.y[1], J.y_stride, gi, conv1);
+            },
+            [&](const Raw6 &q, int e, u128(&z)[kOuts]) {
+                const u128 x1 = garner_lean(K, quad_word(q.r[0], e), quad_word(q.r[1], e), quad_word(q.r[2], e));
+                const u128 x2 = garner_lean(K, quad_word(q.r[3], e), quad_word(q.r[4], e), quad_word(q.r[5], e));
+#pragma unroll
+                for (int k = 0; k < kOuts; k++) z[k] = combine(x1, x2, k);
+            });
+    }
 #pragma unroll
     for (int k = 0; k < kOuts; k++) {
-        uint32_t *const row = planes + 3 * k * cs_plane<CS_T>() + t * CS_ROW;
+        uint32_t *const row = planes + 3 * k * Q::PLANE + t * Q::ROW;
         Super S;
         uint64_t cin = 0;
-        if (t < CS_T) super_sum<CS_T, B>(S, row, false, words_value);
+        if (t < T) super_sum<Q, SL, B>(S, row, false, words_value);
         if (t == 0) {
             if (cta) {
                 u128 x[4];
@@ -721,25 +799,27 @@ FFG_DEV_INLINE void crt_lin_super(const GarnerConst &K, const CrtLinJob &J, uint
                 cin = (uint64_t)(k0 + k ? J.gamma[1] : J.gamma[0]) + ((uint64_t)1 << (94 - B)); // gamma + K > 0
             }
         }
-        const uint32_t map = super_resolve<CS_T, B>(S, row, sh.sup, cin, 0);
-        super_store<CS_T, B>(planes + 3 * k * cs_plane<CS_T>(), k0 + k ? J.out[1] : J.out[0], (uint64_t)cta * (CS_T * B / 2), J.len);
+        const uint32_t map = super_resolve<T, Q::W>(S, row, sh.sup, cin, 0);
+        super_store<T, Q::W, Q::ROW>(planes + 3 * k * Q::PLANE, k0 + k ? J.out[1] : J.out[0],
+                                     (uint64_t)cta * CRT_NL_PER_W * B, J.len);
         if (t == 0) J.maps[(size_t)(k0 + k) * ncta + cta] = map;
     }
     if (ncta > 1 && last_cta(J.ticket, ncta * gridDim.y)) {
         for (int q = 0; q < 2; q++)
-            settle_cta(q ? J.out[1] : J.out[0], J.len, CS_T * B / 2, J.maps + (size_t)q * ncta, ncta);
+            settle_cta(q ? J.out[1] : J.out[0], J.len, CRT_NL_PER_W * B, J.maps + (size_t)q * ncta, ncta);
         if (t == 0) *J.ticket = 0;
     }
 }
 
-template <int NT, int kOuts> __global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2) k_crt_lin(GarnerConst K, CrtLinJob J) {
+template <int kOuts>
+__global__ void __launch_bounds__(crt_lin_threads<kOuts>(), kOuts == 1 ? 2 : 4) k_crt_lin(GarnerConst K, CrtLinJob J) {
     extern __shared__ __align__(16) uint32_t cs_rows[];
     __shared__ CrtShared sh;
     switch (J.width) {
-    case 32: crt_lin_super<NT, 32, kOuts>(K, J, cs_rows, sh); return;
-    case 33: crt_lin_super<NT, 33, kOuts>(K, J, cs_rows, sh); return;
-    case 34: crt_lin_super<NT, 34, kOuts>(K, J, cs_rows, sh); return;
-    default: crt_lin_super<NT, 35, kOuts>(K, J, cs_rows, sh); return;
+    case 32: crt_lin_super<32, kOuts>(K, J, cs_rows, sh); return;
+    case 33: crt_lin_super<33, kOuts>(K, J, cs_rows, sh); return;
+    case 34: crt_lin_super<34, kOuts>(K, J, cs_rows, sh); return;
+    default: crt_lin_super<35, kOuts>(K, J, cs_rows, sh); return;
     }
 }
 
@@ -759,16 +839,16 @@ static uint32_t crt_lin_split_max() {
 cudaError_t launch_crt_lin(const CrtLinJob &J, cudaStream_t st) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(k_crt_lin<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 1));
-        if (!e) e = cudaFuncSetAttribute(k_crt_lin<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)super_smem(CS_T, 2));
+        cudaError_t e = cudaFuncSetAttribute(k_crt_lin<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * kShortSmem));
+        if (!e) e = cudaFuncSetAttribute(k_crt_lin<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * kBatchSmem));
         if (e) return e;
         configured = true;
     }
     if (J.width < 32 || J.width > 35 || J.alpha[0] <= 0 || J.alpha[1] <= 0) return cudaErrorInvalidValue;
     const uint32_t ncta = crt_ctas(J.len, J.width);
     prof_begin(PK_CRT, st);
-    if (ncta <= crt_lin_split_max()) k_crt_lin<256, 1><<<dim3(ncta, 2), 256, super_smem(CS_T, 1), st>>>(garner_const(), J);
-    else k_crt_lin<128, 2><<<dim3(ncta, 1), 128, super_smem(CS_T, 2), st>>>(garner_const(), J);
+    if (ncta <= crt_lin_split_max()) k_crt_lin<1><<<dim3(ncta, 2), 512, 2 * kShortSmem, st>>>(garner_const(), J);
+    else k_crt_lin<2><<<dim3(ncta, 1), 128, 2 * kBatchSmem, st>>>(garner_const(), J);
     prof_end(PK_CRT, st, 12.0 * (double)(J.conv[0] + J.conv[1]) + 16.0 * (double)J.len);
     return cudaGetLastError();
 }
