@@ -47,7 +47,7 @@ static uint32_t shoup_q(uint32_t w, uint32_t p) { return (uint32_t)(((uint64_t)w
 static uint32_t to_mont(uint32_t x, uint32_t p) { return (uint32_t)(((uint64_t)x << 32) % p); }
 static uint32_t mulm(uint32_t a, uint32_t b, uint32_t p) { return (uint32_t)((uint64_t)a * b % p); }
 
-GarnerConst garner_const() {
+static GarnerConst garner_make() {
     GarnerConst K;
     for (int i = 0; i < 3; i++) K.p[i] = kP[i];
     K.i12 = inv_mod(kP[0] % kP[1], kP[1]);
@@ -57,6 +57,11 @@ GarnerConst garner_const() {
     K.i23 = inv_mod(kP[1] % kP[2], kP[2]);
     K.i23s = shoup_q(K.i23, kP[2]);
     K.p12 = (uint64_t)kP[0] * kP[1];
+    return K;
+}
+// Made once: three modular inverses a launch were microseconds of host time.
+GarnerConst garner_const() {
+    static const GarnerConst K = garner_make();
     return K;
 }
 
@@ -458,14 +463,30 @@ int plan_select(uint64_t bits_a, uint64_t bits_b, int square, ffg_plan *pl) {
     return FFG_OK;
 }
 
-// 2^32 / L mod p as Shoup pairs (undoes the pointwise 2^-32 and the inverse's L).
+// 2^32 / L mod p as Shoup pairs (undoes the pointwise 2^-32 and the inverse's L);
+// kept per length L = 2^lg or 3 2^lg (two modular inverses a prime; called under
+// the layer's lock).
 void scale_consts(uint64_t L, uint32_t *scl, uint32_t *scls) {
+    struct Scale {
+        uint64_t L;
+        uint32_t scl[3], scls[3];
+    };
+    static Scale kept[64][2]; // by lg, radix-3 factor
+    Scale &S = kept[__builtin_ctzll(L) & 63][L & (L - 1) ? 1 : 0];
+    if (S.L == L) {
+        memcpy(scl, S.scl, sizeof S.scl);
+        memcpy(scls, S.scls, sizeof S.scls);
+        return;
+    }
     for (int k = 0; k < 3; k++) {
         uint32_t p = kP[k];
         uint32_t v = mulm((uint32_t)((1ull << 32) % p), inv_mod((uint32_t)(L % p), p), p);
         scl[k] = v;
         scls[k] = shoup_q(v, p);
     }
+    S.L = L;
+    memcpy(S.scl, scl, sizeof S.scl);
+    memcpy(S.scls, scls, sizeof S.scls);
 }
 
 // ---------------------------------------------------------------- multiply
