@@ -92,6 +92,7 @@ constexpr uint32_t kColThreads = 512; // at most; 64 registers each, 32 warps an
 
 template <int RN, bool R3>
 __global__ void __launch_bounds__(kColThreads, 2) k_col_fwd2(Primes3 P3, FourStep G, FSJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ FSJob J;
     if (threadIdx.x == 0) {
@@ -153,6 +154,7 @@ FFG_DEV_INLINE void col_inv2_body(const PrimeDev &P, const FourStep &G, const FS
 
 template <int RN, bool R3>
 __global__ void __launch_bounds__(kColThreads, 2) k_col_inv2(Primes3 P3, FourStep G, FSJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ FSJob J;
     if (threadIdx.x == 0) J = jobs.ext ? jobs.ext[blockIdx.z] : jobs.j[blockIdx.z < FFG_FS_JOBS ? blockIdx.z : 0];
@@ -204,8 +206,8 @@ static cudaError_t launch_col2_t(bool fwd, const Primes3 &P3, const FourStep &G,
     uint32_t threads = groups < tmax ? groups : tmax;
     threads = threads < 64 ? 64 : threads & ~31u;
     threads -= threads % G.wc;
-    if (fwd) k_col_fwd2<RN, R3><<<grid, threads, col2_smem(G), st>>>(P3, G, jobs);
-    else k_col_inv2<RN, R3><<<grid, threads, col2_smem(G), st>>>(P3, G, jobs);
+    if (fwd) launch_after(k_col_fwd2<RN, R3>, grid, threads, col2_smem(G), st, P3, G, jobs);
+    else launch_after(k_col_inv2<RN, R3>, grid, threads, col2_smem(G), st, P3, G, jobs);
     return cudaGetLastError();
 }
 

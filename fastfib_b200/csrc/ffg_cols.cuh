@@ -61,7 +61,7 @@ FFG_DEV_INLINE ColSrc col_src(const uint64_t *limbs, uint64_t ns, uint64_t cs, u
 template <bool W32> struct DigitRaw;
 template <> struct DigitRaw<true> {
     uint32_t v;
-    FFG_DEV_INLINE void fetch(const ColSrc &S, uint32_t i) { v = i < S.cs ? __ldg(S.src + i) : 0u; }
+    FFG_DEV_INLINE void fetch(const ColSrc &S, uint32_t i) { v = i < S.cs ? S.src[i] : 0u; }
     template <int PI> FFG_DEV_INLINE uint32_t residue(const ColSrc &, uint32_t, const PrimeDev &) const {
         constexpr uint32_t p = kPrimeC[PI];
         uint32_t l = v;
@@ -74,9 +74,9 @@ template <> struct DigitRaw<false> {
     FFG_DEV_INLINE void fetch(const ColSrc &S, uint32_t i) {
         const uint32_t bit = S.sft + i * S.w, q = bit >> 5;
         const bool ok = i < S.cs;
-        a = ok && q < S.nw ? __ldg(S.src + q) : 0u;
-        b = ok && q + 1 < S.nw ? __ldg(S.src + q + 1) : 0u;
-        c = ok && (bit & 31) + S.w > 64 && q + 2 < S.nw ? __ldg(S.src + q + 2) : 0u;
+        a = ok && q < S.nw ? S.src[q] : 0u;
+        b = ok && q + 1 < S.nw ? S.src[q + 1] : 0u;
+        c = ok && (bit & 31) + S.w > 64 && q + 2 < S.nw ? S.src[q + 2] : 0u;
     }
     template <int PI> FFG_DEV_INLINE uint32_t residue(const ColSrc &S, uint32_t i, const PrimeDev &P) const {
         constexpr uint32_t p = kPrimeC[PI];

@@ -85,6 +85,7 @@ FFG_DEV_INLINE void conv2_body(const PrimeDev &P, const ConvJob &J, uint32_t *sm
 
 template <int RN, bool R3, bool SQ>
 __global__ void __launch_bounds__(kConvThreads, 2) k_conv2(Primes3 P3, ConvJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ ConvJob J;
     if (threadIdx.x == 0) J = jobs.ext ? jobs.ext[blockIdx.x] : jobs.j[blockIdx.x < FFG_CONV_JOBS ? blockIdx.x : 0];
@@ -118,7 +119,7 @@ static cudaError_t launch_conv2_t(const Primes3 &P3, const ConvJobs &jobs, uint3
     // a thread per 16 words of every operand
     constexpr uint32_t want = (SQ ? 1 : 2) * Q::NBLK * (Q::R / 16);
     constexpr uint32_t threads = want < 32 ? 32 : want > kConvThreads ? kConvThreads : (want + 31) & ~31u;
-    k_conv2<RN, R3, SQ><<<dim3(njobs, 3), threads, sm, st>>>(P3, jobs);
+    launch_after(k_conv2<RN, R3, SQ>, dim3(njobs, 3), threads, sm, st, P3, jobs);
     return cudaGetLastError();
 }
 

@@ -91,6 +91,7 @@ FFG_DEV_INLINE void column_sum(const uint64_t *Xlo, const uint32_t *Xhi, int32_t
 }
 
 __global__ void __launch_bounds__(CRT_THREADS) k_crt_narrow(GarnerConst K, CrtJob J) {
+    after_previous();
     const uint32_t cta = blockIdx.x;
     extern __shared__ __align__(16) unsigned char sm[];
     uint64_t *Xlo = (uint64_t *)sm;                              // CRT_COEF + halo
@@ -501,7 +502,7 @@ struct Raw3 {
 FFG_DEV_INLINE void ld_residues(uint4 *r, const uint32_t *y, uint64_t stride, int64_t gi, uint64_t conv) {
     const bool in = gi >= 0 && (uint64_t)gi < conv;
 #pragma unroll
-    for (int k = 0; k < 3; k++) r[k] = in ? __ldg((const uint4 *)(y + k * stride + gi)) : make_uint4(0, 0, 0, 0);
+    for (int k = 0; k < 3; k++) r[k] = in ? *(const uint4 *)(y + k * stride + gi) : make_uint4(0, 0, 0, 0);
     if (in && (uint64_t)gi + 4 > conv) {
         const uint32_t n = (uint32_t)(conv - (uint64_t)gi); // 1 .. 3 words
 #pragma unroll
@@ -589,6 +590,7 @@ template <CrtForm F> FFG_DEV_INLINE void crt_any(const GarnerConst &K, const Crt
 
 template <CrtForm F>
 __global__ void __launch_bounds__(crt_threads<F>(), F == CF_BATCH ? 6 : (F == CF_SHORT ? 3 : 2)) k_crt(GarnerConst K, CrtJob J) {
+    after_previous();
     crt_any<F>(K, J, blockIdx.x);
 }
 
@@ -598,6 +600,7 @@ struct CrtPair {
     CrtJob j[2];
 };
 __global__ void __launch_bounds__(256, 3) k_crt_pair(GarnerConst K, CrtPair P) {
+    after_previous();
     const CrtJob J = blockIdx.y ? P.j[1] : P.j[0];
     if (blockIdx.x >= crt_ctas_dev(J.nlimbs, J.width)) return;
     crt_any<CF_SHORT>(K, J, blockIdx.x);
@@ -608,6 +611,7 @@ __global__ void __launch_bounds__(256, 3) k_crt_pair(GarnerConst K, CrtPair P) {
 // CTA counts), found by binary search.
 __global__ void __launch_bounds__(128, 6) k_crt_flat(GarnerConst K, const CrtJob *__restrict__ jobs,
                                                             const uint32_t *__restrict__ first, uint32_t count) {
+    after_previous();
     const uint32_t b = blockIdx.x;
     uint32_t lo = 0, hi = count; // invariant: first[lo] <= b < first[hi]
     while (hi - lo > 1) {
@@ -660,10 +664,10 @@ cudaError_t launch_crt(const Primes3 &P3, const CrtJob &J, cudaStream_t st) {
     if (e0) return e0;
     const uint32_t ncta = crt_ctas(J.nlimbs, J.width);
     prof_begin(PK_CRT, st);
-    if (J.width < 32) k_crt_narrow<<<ncta, CRT_THREADS, crt_smem(), st>>>(garner_const(), J);
-    else if (ncta <= kCrtShortCtas) k_crt<CF_SHORT><<<ncta, 256, kShortSmem, st>>>(garner_const(), J);
-    else if (ncta <= kCrtBigCtas) k_crt<CF_BATCH><<<ncta, 128, kBatchSmem, st>>>(garner_const(), J);
-    else k_crt<CF_LONG><<<(ncta + 3) / 4, 256, kLongSmem, st>>>(garner_const(), J);
+    if (J.width < 32) launch_after(k_crt_narrow, ncta, CRT_THREADS, crt_smem(), st, garner_const(), J);
+    else if (ncta <= kCrtShortCtas) launch_after(k_crt<CF_SHORT>, ncta, 256, kShortSmem, st, garner_const(), J);
+    else if (ncta <= kCrtBigCtas) launch_after(k_crt<CF_BATCH>, ncta, 128, kBatchSmem, st, garner_const(), J);
+    else launch_after(k_crt<CF_LONG>, (ncta + 3) / 4, 256, kLongSmem, st, garner_const(), J);
     prof_end(PK_CRT, st, 12.0 * (double)J.conv + 8.0 * (double)J.nlimbs);
     return cudaGetLastError();
 }
@@ -683,7 +687,7 @@ cudaError_t launch_crt_pair(const CrtJob *jobs, uint32_t count, cudaStream_t st)
     double bytes = 0;
     for (int i = 0; i < 2; i++) bytes += 12.0 * (double)jobs[i].conv + 8.0 * (double)jobs[i].nlimbs;
     prof_begin(PK_CRT, st);
-    k_crt_pair<<<dim3(n0 > n1 ? n0 : n1, 2), 256, kShortSmem, st>>>(garner_const(), P);
+    launch_after(k_crt_pair, dim3(n0 > n1 ? n0 : n1, 2), 256, kShortSmem, st, garner_const(), P);
     prof_end(PK_CRT, st, bytes);
     return cudaGetLastError();
 }
@@ -692,7 +696,7 @@ cudaError_t launch_crt_flat(const CrtJob *d_jobs, const uint32_t *d_first, uint3
                             cudaStream_t st, double bytes) {
     if (!count || !total_ctas) return cudaSuccess;
     prof_begin(PK_CRT, st);
-    k_crt_flat<<<total_ctas, 128, kBatchSmem, st>>>(garner_const(), d_jobs, d_first, count);
+    launch_after(k_crt_flat, total_ctas, 128, kBatchSmem, st, garner_const(), d_jobs, d_first, count);
     prof_end(PK_CRT, st, bytes);
     return cudaGetLastError();
 }
@@ -813,6 +817,7 @@ FFG_DEV_INLINE void crt_lin_super(const GarnerConst &K, const CrtLinJob &J, uint
 
 template <int kOuts>
 __global__ void __launch_bounds__(crt_lin_threads<kOuts>(), kOuts == 1 ? 2 : 4) k_crt_lin(GarnerConst K, CrtLinJob J) {
+    after_previous();
     extern __shared__ __align__(16) uint32_t cs_rows[];
     __shared__ CrtShared sh;
     switch (J.width) {
@@ -847,8 +852,8 @@ cudaError_t launch_crt_lin(const CrtLinJob &J, cudaStream_t st) {
     if (J.width < 32 || J.width > 35 || J.alpha[0] <= 0 || J.alpha[1] <= 0) return cudaErrorInvalidValue;
     const uint32_t ncta = crt_ctas(J.len, J.width);
     prof_begin(PK_CRT, st);
-    if (ncta <= crt_lin_split_max()) k_crt_lin<1><<<dim3(ncta, 2), 512, 2 * kShortSmem, st>>>(garner_const(), J);
-    else k_crt_lin<2><<<dim3(ncta, 1), 128, 2 * kBatchSmem, st>>>(garner_const(), J);
+    if (ncta <= crt_lin_split_max()) launch_after(k_crt_lin<1>, dim3(ncta, 2), 512, 2 * kShortSmem, st, garner_const(), J);
+    else launch_after(k_crt_lin<2>, dim3(ncta, 1), 128, 2 * kBatchSmem, st, garner_const(), J);
     prof_end(PK_CRT, st, 12.0 * (double)(J.conv[0] + J.conv[1]) + 16.0 * (double)J.len);
     return cudaGetLastError();
 }
@@ -887,6 +892,7 @@ FFG_DEV_INLINE void school_col(const SchoolJob &J, int64_t j, uint64_t &t0, uint
 FFG_DEV_INLINE void school_block(const SchoolJob &J);
 
 __global__ void __launch_bounds__(SCHOOL_THREADS) k_school(const SchoolJob *__restrict__ jobs) {
+    after_previous();
     const SchoolJob J = jobs[blockIdx.y];
     if (blockIdx.x >= school_ctas(J.nlimbs)) return;
     school_block(J);
@@ -898,6 +904,7 @@ struct SchoolPair {
     SchoolJob j[2];
 };
 __global__ void __launch_bounds__(SCHOOL_THREADS) k_school_pair(SchoolPair P) {
+    after_previous();
     const SchoolJob &J = P.j[blockIdx.y];
     if (blockIdx.x >= school_ctas(J.nlimbs)) return;
     school_block(J);
@@ -951,7 +958,7 @@ cudaError_t launch_school_pair(const SchoolJob *jobs, uint32_t count, cudaStream
         bytes += 8.0 * (double)(jobs[i].na + jobs[i].nb + jobs[i].nlimbs);
     }
     prof_begin(PK_SCHOOL, st);
-    k_school_pair<<<dim3(mx, count), SCHOOL_THREADS, 0, st>>>(P);
+    launch_after(k_school_pair, dim3(mx, count), SCHOOL_THREADS, 0, st, P);
     prof_end(PK_SCHOOL, st, bytes);
     return cudaGetLastError();
 }
@@ -968,6 +975,7 @@ constexpr uint32_t SQ_TPC = 4; // threads per column
 __host__ __device__ uint32_t school_sq_ctas(uint64_t nlimbs) { return (uint32_t)((nlimbs + SQ_NL - 1) / SQ_NL); }
 
 __global__ void __launch_bounds__(SCHOOL_THREADS) k_school_sq_pair(SchoolPair Pr) {
+    after_previous();
     const SchoolJob &J = blockIdx.y ? Pr.j[1] : Pr.j[0];
     const uint32_t ncta = school_sq_ctas(J.nlimbs);
     if (blockIdx.x >= ncta) return;
@@ -990,7 +998,7 @@ __global__ void __launch_bounds__(SCHOOL_THREADS) k_school_sq_pair(SchoolPair Pr
         if (j >= 1 && j <= 2 * n - 3) {
             const int64_t ilo = j - n + 1 > 0 ? j - n + 1 : 0, ihi = (j - 1) / 2; // i < j - i
             for (int64_t i = ilo + part; i <= ihi; i += SQ_TPC) {
-                const u128 pr = (u128)__ldg(&a[i]) * __ldg(&a[j - i]);
+                const u128 pr = (u128)a[i] * a[j - i];
                 const uint64_t l = (uint64_t)pr, h = (uint64_t)(pr >> 64);
                 t0 += l;
                 const uint64_t hh = h + (t0 < l);
@@ -1020,7 +1028,7 @@ __global__ void __launch_bounds__(SCHOOL_THREADS) k_school_sq_pair(SchoolPair Pr
         t1 = (t1 << 1) | (t0 >> 63);
         t0 <<= 1;
         if (j >= 0 && j <= 2 * n - 2 && (j & 1) == 0) {
-            const uint64_t x = __ldg(&a[j / 2]);
+            const uint64_t x = a[j / 2];
             const u128 sq = (u128)x * x;
             const uint64_t l = (uint64_t)sq, h = (uint64_t)(sq >> 64);
             t0 += l;
@@ -1066,7 +1074,7 @@ cudaError_t launch_school_sq_pair(const SchoolJob *jobs, uint32_t count, cudaStr
         bytes += 8.0 * (double)(jobs[i].na + jobs[i].nlimbs);
     }
     prof_begin(PK_SCHOOL, st);
-    k_school_sq_pair<<<dim3(mx, count), SCHOOL_THREADS, 0, st>>>(P);
+    launch_after(k_school_sq_pair, dim3(mx, count), SCHOOL_THREADS, 0, st, P);
     prof_end(PK_SCHOOL, st, bytes);
     return cudaGetLastError();
 }
@@ -1075,7 +1083,7 @@ cudaError_t launch_school_batch(const SchoolJob *d_jobs, uint32_t count, uint32_
                                 double bytes) {
     if (!count) return cudaSuccess;
     prof_begin(PK_SCHOOL, st);
-    k_school<<<dim3(max_ctas, count), SCHOOL_THREADS, 0, st>>>(d_jobs);
+    launch_after(k_school, dim3(max_ctas, count), SCHOOL_THREADS, 0, st, d_jobs);
     prof_end(PK_SCHOOL, st, bytes);
     return cudaGetLastError();
 }
@@ -1107,6 +1115,7 @@ FFG_DEV_INLINE void lin_colsum(const LinJob &J, uint32_t k, uint64_t j, uint64_t
 }
 
 __global__ void __launch_bounds__(LIN_THREADS) k_lin(LinJob J) {
+    after_previous();
     __shared__ uint64_t lo[LIN_NL];
     __shared__ uint32_t hi[LIN_NL];
     __shared__ uint32_t gG[LIN_NL / 32], gP[LIN_NL / 32], gin[LIN_NL / 32];
@@ -1118,8 +1127,8 @@ __global__ void __launch_bounds__(LIN_THREADS) k_lin(LinJob J) {
 #pragma unroll
     for (int r = 0; r < PER; r++) {
         const uint64_t j = j0 + threadIdx.x + r * LIN_THREADS;
-        xs[r] = j < J.n1 ? __ldg(&J.s1[j]) : 0;
-        ys[r] = j < J.n2 ? __ldg(&J.s2[j]) : 0;
+        xs[r] = j < J.n1 ? J.s1[j] : 0;
+        ys[r] = j < J.n2 ? J.s2[j] : 0;
     }
     uint64_t xp = 0, yp = 0; // limb j0 - 1, for the carry into the CTA's first limb
     if (threadIdx.x == 0 && j0 > 0) {
@@ -1158,7 +1167,7 @@ __global__ void __launch_bounds__(LIN_THREADS) k_lin(LinJob J) {
 cudaError_t launch_lin(const LinJob &J, cudaStream_t st) {
     const uint32_t ncta = lin_ctas(J.len);
     prof_begin(PK_LIN, st);
-    k_lin<<<ncta, LIN_THREADS, 0, st>>>(J);
+    launch_after(k_lin, ncta, LIN_THREADS, 0, st, J);
     prof_end(PK_LIN, st, 8.0 * (double)(J.n1 + J.n2) + 8.0 * (double)J.len * J.nout);
     return cudaGetLastError();
 }

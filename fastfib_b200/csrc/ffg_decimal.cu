@@ -31,6 +31,7 @@ typedef unsigned __int128 u128;
 // ------------------------------------------------------------------ shift
 
 __global__ void __launch_bounds__(256) k_shift_batch(const ShiftJob *__restrict__ jobs) {
+    after_previous();
     const ShiftJob J = jobs[blockIdx.y];
     const uint64_t w = J.shift >> 6;
     const uint32_t b = (uint32_t)(J.shift & 63);
@@ -49,7 +50,7 @@ cudaError_t launch_shift_batch(const ShiftJob *d_jobs, uint32_t count, uint64_t 
     for (uint32_t base = 0; base < count; base += 65535) {
         const uint32_t cnt = count - base < 65535 ? count - base : 65535;
         prof_begin(PK_LIN, st);
-        k_shift_batch<<<dim3((uint32_t)blocks, cnt), 256, 0, st>>>(d_jobs + base);
+        launch_after(k_shift_batch, dim3((uint32_t)blocks, cnt), 256, 0, st, d_jobs + base);
         prof_end(PK_LIN, st, 16.0 * (double)max_out * cnt);
         cudaError_t e = cudaGetLastError();
         if (e) return e;
@@ -101,7 +102,7 @@ FFG_DEV_INLINE void comb_colsum(const CombJob &J, const CombTerms &T, uint64_t j
 #pragma unroll
     for (int t = 0; t < 3; t++) {
         if (!T.mag[t]) continue;
-        uint64_t v = j < J.n[t] ? __ldg(&J.src[t][j]) : 0;
+        uint64_t v = j < J.n[t] ? J.src[t][j] : 0;
         if (T.neg[t]) v = ~v;
         acc += (u128)v * T.mag[t];
     }
@@ -110,6 +111,7 @@ FFG_DEV_INLINE void comb_colsum(const CombJob &J, const CombTerms &T, uint64_t j
 }
 
 __global__ void __launch_bounds__(COMB_THREADS) k_comb_batch(const CombJob *__restrict__ jobs, uint32_t nl) {
+    after_previous();
     __shared__ uint64_t lo[COMB_NL];
     __shared__ uint32_t hi[COMB_NL];
     __shared__ uint32_t gG[COMB_NL / 32], gP[COMB_NL / 32], gin[COMB_NL / 32];
@@ -158,7 +160,7 @@ cudaError_t launch_comb_batch(const CombJob *d_jobs, uint32_t count, uint64_t ma
     for (uint32_t base = 0; base < count; base += 65535) {
         const uint32_t cnt = count - base < 65535 ? count - base : 65535;
         prof_begin(PK_LIN, st);
-        k_comb_batch<<<dim3(ctas, cnt), threads, 0, st>>>(d_jobs + base, nl);
+        launch_after(k_comb_batch, dim3(ctas, cnt), threads, 0, st, d_jobs + base, nl);
         prof_end(PK_LIN, st, 32.0 * (double)max_len * cnt);
         cudaError_t e = cudaGetLastError();
         if (e) return e;
@@ -177,6 +179,7 @@ FFG_DEV_INLINE uint64_t window64(const uint64_t *x, uint64_t n, uint64_t e) {
 }
 
 __global__ void __launch_bounds__(256) k_khat_batch(const KhatJob *__restrict__ jobs, uint32_t count) {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const KhatJob J = jobs[i];
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(256) k_khat_batch(const KhatJob *__restrict__ 
 cudaError_t launch_khat_batch(const KhatJob *d_jobs, uint32_t count, cudaStream_t st) {
     if (!count) return cudaSuccess;
     prof_begin(PK_LIN, st);
-    k_khat_batch<<<(count + 255) / 256, 256, 0, st>>>(d_jobs, count);
+    launch_after(k_khat_batch, (count + 255) / 256, 256, 0, st, d_jobs, count);
     prof_end(PK_LIN, st, 48.0 * count);
     return cudaGetLastError();
 }
@@ -227,6 +230,7 @@ FFG_DEV_INLINE uint64_t div_2by1(uint64_t u1, uint64_t u0, uint64_t v, uint64_t 
 
 __global__ void __launch_bounds__(32) k_leaf_digits(const LeafJob *__restrict__ jobs, uint32_t count, uint32_t chunks,
                                                       uint64_t v, char *out) {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const LeafJob J = jobs[i];
@@ -254,7 +258,7 @@ cudaError_t launch_leaf_digits(const LeafJob *d_jobs, uint32_t count, uint32_t c
     prof_begin(PK_LIN, st);
     // one thread a leaf, one warp a CTA: the leaves' serial divisions spread
     // over every SM instead of a quarter as many
-    k_leaf_digits<<<(count + 31) / 32, 32, 0, st>>>(d_jobs, count, chunks, v, d_out);
+    launch_after(k_leaf_digits, (count + 31) / 32, 32, 0, st, d_jobs, count, chunks, v, d_out);
     prof_end(PK_LIN, st, (double)count * chunks * 19);
     return cudaGetLastError();
 }
@@ -265,6 +269,7 @@ cudaError_t launch_leaf_digits(const LeafJob *d_jobs, uint32_t count, uint32_t c
 // stride) and stops at its first find, the block keeps its minimum, and one
 // atomic per block publishes it.  d is 16-byte aligned.
 __global__ void __launch_bounds__(256) k_first_nonzero(const char *d, uint64_t n, unsigned long long *first) {
+    after_previous();
     __shared__ unsigned long long best;
     if (threadIdx.x == 0) best = ~0ull;
     __syncthreads();
@@ -293,7 +298,7 @@ __global__ void __launch_bounds__(256) k_first_nonzero(const char *d, uint64_t n
 
 cudaError_t launch_first_nonzero(const char *d, uint64_t n, unsigned long long *d_first, cudaStream_t st) {
     const uint64_t blocks = (n + 16 * 256 - 1) / (16 * 256);
-    k_first_nonzero<<<(uint32_t)(blocks < 592 ? (blocks ? blocks : 1) : 592), 256, 0, st>>>(d, n, d_first);
+    launch_after(k_first_nonzero, (uint32_t)(blocks < 592 ? (blocks ? blocks : 1) : 592), 256, 0, st, d, n, d_first);
     return cudaGetLastError();
 }
 

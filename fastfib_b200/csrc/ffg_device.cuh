@@ -139,14 +139,19 @@ FFG_DEV_INLINE uint32_t tw_mont(const PrimeDev &P, uint64_t E) {
     return mont(lo, hi, P.p, P.pinv); // (ω^El 2^32)(ω^Eh 2^32) 2^-32
 }
 
+// First in every kernel that launch_after starts: waits until the kernel before it in
+// the stream has completed and its writes are visible.  What that kernel wrote is read
+// with plain loads after this, not through the read-only path.
+FFG_DEV_INLINE void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // b-bit digit i of the limb array a (na limbs), zero past the end: the
 // reference's Src reader (src/ntt_kernels.c:29-74).
 FFG_DEV_INLINE uint64_t digit_at(const uint64_t *__restrict__ a, uint64_t na, uint64_t i, uint32_t b) {
     uint64_t bit = i * b, q = bit >> 6;
     uint32_t off = (uint32_t)(bit & 63);
     if (q >= na) return 0;
-    uint64_t lo = __ldg(&a[q]);
-    uint64_t hi = (off + b > 64 && q + 1 < na) ? __ldg(&a[q + 1]) : 0;
+    uint64_t lo = a[q];
+    uint64_t hi = (off + b > 64 && q + 1 < na) ? a[q + 1] : 0;
     uint64_t v = off ? (lo >> off) | (hi << (64 - off)) : lo;
     return v & ((1ull << b) - 1);
 }

@@ -361,8 +361,8 @@ FFG_DEV_INLINE void tile_digits(uint32_t *__restrict__ smem, uint32_t stride, co
             const uint64_t bit = (off + i) * w, q = bit >> 6;
             sh[b] = (uint32_t)(bit & 63);
             const bool ok = it < items && i < cs;
-            lo[b] = ok && q < ns ? __ldg(&src[q]) : 0;
-            hi[b] = ok && sh[b] + w > 64 && q + 1 < ns ? __ldg(&src[q + 1]) : 0;
+            lo[b] = ok && q < ns ? src[q] : 0;
+            hi[b] = ok && sh[b] + w > 64 && q + 1 < ns ? src[q + 1] : 0;
         }
 #pragma unroll
         for (int b = 0; b < kB; b++) {

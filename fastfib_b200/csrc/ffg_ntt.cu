@@ -78,6 +78,7 @@ FFG_DEV_INLINE void conv_small_body(const PrimeDev &P, const ConvJob &J, uint32_
 }
 
 __global__ void __launch_bounds__(kLineThreads, kLineMinBlocks) k_conv_small(Primes3 P3, ConvJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ ConvJob J;
     job_to_smem<ConvJobs, ConvJob, FFG_CONV_JOBS>(jobs, blockIdx.x, &J);
@@ -125,6 +126,7 @@ FFG_DEV_INLINE void col_fwd_body(const PrimeDev &P, const FourStep &G, const FSJ
 }
 
 __global__ void __launch_bounds__(kLineThreads, kLineMinBlocks) k_col_fwd(Primes3 P3, FourStep G, FSJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ FSJob J;
     job_to_smem<FSJobs, FSJob, FFG_FS_JOBS>(jobs, G.square ? blockIdx.z : (blockIdx.z >> 1), &J);
@@ -196,6 +198,7 @@ FFG_DEV_INLINE void row_body(const PrimeDev &P, const FourStep &G, const FSJob &
 }
 
 __global__ void __launch_bounds__(kLineThreads, kLineMinBlocks) k_row_conv(Primes3 P3, FourStep G, FSJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ FSJob J;
     job_to_smem<FSJobs, FSJob, FFG_FS_JOBS>(jobs, blockIdx.z, &J);
@@ -225,6 +228,7 @@ FFG_DEV_INLINE void col_inv_body(const PrimeDev &P, const FourStep &G, const FSJ
 }
 
 __global__ void __launch_bounds__(kLineThreads, kLineMinBlocks) k_col_inv(Primes3 P3, FourStep G, FSJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ FSJob J;
     job_to_smem<FSJobs, FSJob, FFG_FS_JOBS>(jobs, blockIdx.z, &J);
@@ -271,7 +275,7 @@ cudaError_t launch_conv_small(const Primes3 &P3, const ConvJobs &jobs, uint32_t 
     if (conv2_ok(n, r3)) {
         e = launch_conv2(P3, jobs, njobs, n, r3, square, st);
     } else {
-        k_conv_small<<<dim3(njobs, 3, 1), 256, small_smem_bytes((r3 ? 3u : 1u) << n, square), st>>>(P3, jobs);
+        launch_after(k_conv_small, dim3(njobs, 3, 1), 256, small_smem_bytes((r3 ? 3u : 1u) << n, square), st, P3, jobs);
         e = cudaGetLastError();
     }
     prof_end(PK_CONV_SMALL, st, bytes);
@@ -317,7 +321,7 @@ cudaError_t launch_four_step(const Primes3 &P3, const FourStep &G, const FSJobs 
     if (col2) {
         e = launch_col2(true, P3, G, jobs, njobs * nops, st);
     } else {
-        k_col_fwd<<<dim3(tiles, G.nprimes, njobs * nops), 256, sm_col, st>>>(P3, G, jobs);
+        launch_after(k_col_fwd, dim3(tiles, G.nprimes, njobs * nops), 256, sm_col, st, P3, G, jobs);
         e = cudaGetLastError();
     }
     prof_end(PK_COL_FWD, st, res * nops + limb_bytes);
@@ -326,7 +330,7 @@ cudaError_t launch_four_step(const Primes3 &P3, const FourStep &G, const FSJobs 
     if (g_row2 && row2_ok(G)) {
         e = launch_row2(P3, G, jobs, njobs, st);
     } else {
-        k_row_conv<<<dim3(G.R, G.nprimes, njobs), 256, sm_row, st>>>(P3, G, jobs);
+        launch_after(k_row_conv, dim3(G.R, G.nprimes, njobs), 256, sm_row, st, P3, G, jobs);
         e = cudaGetLastError();
     }
     prof_end(PK_ROW_CONV, st, res * (nops + 1));
@@ -335,7 +339,7 @@ cudaError_t launch_four_step(const Primes3 &P3, const FourStep &G, const FSJobs 
     if (col2) {
         e = launch_col2(false, P3, G, jobs, njobs, st);
     } else {
-        k_col_inv<<<dim3(tiles, G.nprimes, njobs), 256, sm_col, st>>>(P3, G, jobs);
+        launch_after(k_col_inv, dim3(tiles, G.nprimes, njobs), 256, sm_col, st, P3, G, jobs);
         e = cudaGetLastError();
     }
     prof_end(PK_COL_INV, st, res * 2);
@@ -376,7 +380,7 @@ cudaError_t launch_split_forward(const Primes3 &P3, FourStep G, const FSJobs &jo
     if (g_col2 && col2_ok(G)) {
         e = launch_col2(true, P3, G, jobs, njobs, st);
     } else {
-        k_col_fwd<<<dim3(tiles, G.nprimes, njobs), 256, sm_col, st>>>(P3, G, jobs);
+        launch_after(k_col_fwd, dim3(tiles, G.nprimes, njobs), 256, sm_col, st, P3, G, jobs);
         e = cudaGetLastError();
     }
     prof_end(PK_COL_FWD, st, res + limb_bytes);
@@ -385,7 +389,7 @@ cudaError_t launch_split_forward(const Primes3 &P3, FourStep G, const FSJobs &jo
     if (g_row2 && row2_ok(G)) {
         e = launch_row2(P3, G, jobs, njobs, st);
     } else {
-        k_row_conv<<<dim3(G.R, G.nprimes, njobs), 256, sm_row, st>>>(P3, G, jobs);
+        launch_after(k_row_conv, dim3(G.R, G.nprimes, njobs), 256, sm_row, st, P3, G, jobs);
         e = cudaGetLastError();
     }
     prof_end(PK_ROW_CONV, st, res * 2);
@@ -408,7 +412,7 @@ cudaError_t launch_split_piece(const Primes3 &P3, FourStep G, const FSJob &job, 
     if (g_row2 && row2_ok(G)) {
         e = launch_row2(P3, G, one, 1, st);
     } else {
-        k_row_conv<<<dim3(G.R, G.nprimes, 1), 256, sm_row, st>>>(P3, G, one);
+        launch_after(k_row_conv, dim3(G.R, G.nprimes, 1), 256, sm_row, st, P3, G, one);
         e = cudaGetLastError();
     }
     prof_end(PK_ROW_CONV, st, res * (2.0 * pairs + 1.0));
@@ -417,7 +421,7 @@ cudaError_t launch_split_piece(const Primes3 &P3, FourStep G, const FSJob &job, 
     if (g_col2 && col2_ok(G)) {
         e = launch_col2(false, P3, G, one, 1, st);
     } else {
-        k_col_inv<<<dim3(tiles, G.nprimes, 1), 256, sm_col, st>>>(P3, G, one);
+        launch_after(k_col_inv, dim3(tiles, G.nprimes, 1), 256, sm_col, st, P3, G, one);
         e = cudaGetLastError();
     }
     prof_end(PK_COL_INV, st, res * 3.0);

@@ -120,7 +120,7 @@ enum RowKind { RK_SQUARE, RK_PRODUCT, RK_FORWARD, RK_PIECE };
 FFG_DEV_INLINE void ld16(uint32_t (&x)[16], const uint32_t *p) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const uint4 v = __ldg((const uint4 *)p + k);
+        const uint4 v = ((const uint4 *)p)[k];
         x[4 * k] = v.x, x[4 * k + 1] = v.y, x[4 * k + 2] = v.z, x[4 * k + 3] = v.w;
     }
 }
@@ -268,6 +268,7 @@ FFG_DEV_INLINE void row2_body(const PrimeDev &P, const FourStep &G, const FSJob 
 
 template <int CLG, int KIND>
 __global__ void __launch_bounds__(256, CLG == 13 && KIND == RK_PRODUCT ? 3 : 4) k_row2(Primes3 P3, FourStep G, FSJobs jobs) {
+    after_previous();
     extern __shared__ uint32_t smem[];
     __shared__ FSJob J;
     if (threadIdx.x == 0) J = jobs.ext ? jobs.ext[blockIdx.z] : jobs.j[blockIdx.z < FFG_FS_JOBS ? blockIdx.z : 0];
@@ -305,7 +306,7 @@ static cudaError_t launch_row2_t(const Primes3 &P3, const FourStep &G, const FSJ
     while (rows > 1 && (uint64_t)(G.R / rows) * G.nprimes * njobs < 3 * 148) rows >>= 1;
     while (rows > 1 && G.R % rows) rows >>= 1;
     const size_t sm = (size_t)rows * lines * Q::LS * sizeof(uint32_t);
-    k_row2<CLG, KIND><<<dim3(G.R / rows, G.nprimes, njobs), rows * Q::T, sm, st>>>(P3, G, jobs);
+    launch_after(k_row2<CLG, KIND>, dim3(G.R / rows, G.nprimes, njobs), rows * Q::T, sm, st, P3, G, jobs);
     return cudaGetLastError();
 }
 
