@@ -1088,6 +1088,151 @@ cudaError_t launch_school_batch(const SchoolJob *d_jobs, uint32_t count, uint32_
     return cudaGetLastError();
 }
 
+// k_chain_steps: the doubling chain's first steps, up to STEP_IN limbs of operand, in
+// one launch of one CTA: both squarings, the linear combinations and the carries of
+// every step in shared memory.  As k_school_sq_pair and k_lin a step this short is two
+// launches' latency (chain of F(20 000) 28.0 -> 25.4 us, of F(10^5) 55.4 -> 49.2, of
+// F(10^7) 234 -> 227).  Longer steps are bound by the one SM's multiplier and keep
+// their CTAs: with steps of up to 288 limbs F(10^5) takes 56.7 us.
+//
+// A step on n limbs: columns j and j + n of a square have n / 2 products together, so
+// a thread takes every P-th product of such a pair (neighbours in j: one operand is a
+// broadcast, the other consecutive).  P is what the threads allow, at most 8 (the parts
+// are added by one thread a column).  A column's 192-bit sum
+// t0 + 2^64 t1 + 2^128 t2 gives v_j = t0_j + t1_(j-1) + t2_(j-2) < 3 2^64, and output
+// limb j is alpha v1_j + beta v2_j + 8 (2^64 - 1) >= 0 (beta >= -2): the bias adds
+// 8 (2^(64 N) - 1) over the N limbs, so 8 more at limb 0 takes it out modulo 2^(64 N).
+// Both outputs are resolved as one row with a zero limb behind each, which takes what
+// runs out of the top.
+constexpr uint32_t STEP_THREADS = 1024;
+constexpr uint32_t STEP_ROW = 2 * STEP_IN + 32; // limbs of an output, with at least one of padding
+static_assert(STEP_ROW % 32 == 0 && STEP_ROW >= 2 * STEP_IN + 2 && 2 * STEP_IN <= STEP_THREADS, "outputs and their padding, slots");
+
+struct StepShared {
+    uint64_t lo[2 * STEP_ROW];         // the pair: F(k-1), then F(k)
+    uint64_t p0[2 * STEP_THREADS], p1[2 * STEP_THREADS]; // parts of the columns' sums
+    uint64_t t0[4 * STEP_IN], t1[4 * STEP_IN];       // the columns' sums
+    uint32_t p2[2 * STEP_THREADS], t2[4 * STEP_IN];
+    uint32_t hi[2 * STEP_ROW];
+    uint32_t gG[2 * STEP_ROW / 32], gP[2 * STEP_ROW / 32], gin[2 * STEP_ROW / 32];
+};
+
+__global__ void __launch_bounds__(STEP_THREADS) k_chain_steps(ChainSteps J) {
+    after_previous();
+    extern __shared__ __align__(16) unsigned char step_smem[];
+    StepShared &S = *(StepShared *)step_smem;
+    for (uint32_t j = threadIdx.x; j < 2 * STEP_IN; j += STEP_THREADS) {
+        const bool up = j >= STEP_IN;
+        const uint32_t i = up ? j - STEP_IN : j;
+        S.lo[up ? STEP_ROW + i : i] = i < (up ? J.nk : J.nkm1) ? (up ? J.fk : J.fkm1)[i] : 0;
+    }
+    __syncthreads();
+    uint32_t n = J.nk, odd = J.odd, row = STEP_ROW;
+    for (uint32_t step = 0; step < J.steps; step++) {
+        const uint32_t N = J.n_out[step], bit = J.bits >> step & 1u;
+        // parts: slot (q, p, j) of columns j and j + n of square q (0: F(k), 1: F(k-1))
+        const uint32_t fit = STEP_THREADS / (2 * n), P = fit < 8 ? fit : 8;
+        for (uint32_t s = threadIdx.x; s < 2 * n * P; s += STEP_THREADS) {
+            const uint32_t j = s % n, r = s / n, q = r >= P, p = q ? r - P : r;
+            const uint64_t *a = S.lo + (q ? 0 : row);
+#pragma unroll
+            for (uint32_t half = 0; half < 2; half++) {
+                const uint32_t c = j + half * n, ilo = half ? j + 1 : 0, iend = (c + 1) / 2; // i < c - i
+                uint64_t t0 = 0, t1 = 0, t2 = 0;
+#pragma unroll 2
+                for (uint32_t i = ilo + p; i < iend; i += P) {
+                    const u128 pr = (u128)a[i] * a[c - i];
+                    const u128 sum = (u128)t1 << 64 | t0, acc = sum + pr;
+                    t2 += acc < pr;
+                    t0 = (uint64_t)acc;
+                    t1 = (uint64_t)(acc >> 64);
+                }
+                const uint32_t at = (q * P + p) * 2 * n + c;
+                S.p0[at] = t0;
+                S.p1[at] = t1;
+                S.p2[at] = (uint32_t)t2;
+            }
+        }
+        __syncthreads();
+        // column c of square q: twice its parts, and the middle square
+        for (uint32_t s = threadIdx.x; s < 4 * n; s += STEP_THREADS) {
+            const uint32_t q = s >= 2 * n, c = q ? s - 2 * n : s;
+            u128 acc = 0;
+            uint64_t top = 0;
+            for (uint32_t p = 0; p < P; p++) {
+                const uint32_t at = (q * P + p) * 2 * n + c;
+                const u128 v = (u128)S.p1[at] << 64 | S.p0[at];
+                acc += v;
+                top += S.p2[at] + (acc < v);
+            }
+            top = top << 1 | (uint64_t)(acc >> 127);
+            acc <<= 1;
+            if (!(c & 1)) {
+                const uint64_t x = S.lo[(q ? 0 : row) + c / 2];
+                const u128 sq = (u128)x * x;
+                acc += sq;
+                top += acc < sq;
+            }
+            S.t0[s] = (uint64_t)acc;
+            S.t1[s] = (uint64_t)(acc >> 64);
+            S.t2[s] = (uint32_t)top;
+        }
+        __syncthreads();
+        const int64_t pm2 = odd ? -2 : 2;
+        row = (N + 32) & ~31u; // the outputs' rows: N limbs and at least one of padding
+        for (uint32_t s = threadIdx.x; s < 2 * row; s += STEP_THREADS) {
+            const uint32_t k = s >= row, j = k ? s - row : s;
+            u128 w = 0;
+            if (j < N) {
+                auto column = [&](uint32_t q) { // v_j of square q
+                    const uint32_t b = q * 2 * n;
+                    u128 v = j < 2 * n ? S.t0[b + j] : 0;
+                    if (j >= 1 && j - 1 < 2 * n) v += S.t1[b + j - 1];
+                    if (j >= 2 && j - 2 < 2 * n) v += S.t2[b + j - 2];
+                    return v;
+                };
+                const u128 v1 = column(0), v2 = column(1);
+                // bit: 3 s1 - 2 s2 +- 2 and 4 s1 - s2 +- 2, else s1 + s2 and 3 s1 - 2 s2 +- 2
+                const bool plain = !bit && !k;
+                w = plain ? v1 + v2 : (bit && k ? v1 * 4 - v2 : v1 * 3 - v2 * 2);
+                if (!plain) {
+                    w += (u128)~0ull * 8;
+                    if (j == 0) w += (u128)(uint64_t)(8 + pm2);
+                }
+            }
+            S.lo[s] = (uint64_t)w;
+            S.hi[s] = (uint32_t)(w >> 64);
+        }
+        __syncthreads();
+        cta_resolve(S.lo, S.hi, 0, 2 * row, S.gG, S.gP, S.gin);
+        n = N;
+        odd = bit;
+    }
+    for (uint32_t j = threadIdx.x; j < 2 * n; j += STEP_THREADS) {
+        const bool up = j >= n;
+        const uint32_t i = up ? j - n : j;
+        (up ? J.ok : J.okm1)[i] = S.lo[up ? row + i : i];
+    }
+}
+
+cudaError_t launch_chain_steps(const ChainSteps &J, cudaStream_t st) {
+    if (J.nk < 1 || J.nk > STEP_IN || J.nkm1 > J.nk || J.steps < 1 || J.steps > FFG_CHAIN_STEPS)
+        return cudaErrorInvalidValue;
+    for (uint32_t k = 0, n = J.nk; k < J.steps; n = J.n_out[k++])
+        if (n > STEP_IN || J.n_out[k] < 1 || J.n_out[k] > 2 * n + 1) return cudaErrorInvalidValue;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(k_chain_steps, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(StepShared));
+        if (e) return e;
+        configured = true;
+    }
+    prof_begin(PK_SCHOOL, st);
+    launch_after(k_chain_steps, 1, STEP_THREADS, sizeof(StepShared), st, J);
+    prof_end(PK_SCHOOL, st, 8.0 * (double)(J.nk + J.nkm1 + 2 * J.n_out[J.steps - 1]));
+    return cudaGetLastError();
+}
+
 // ------------------------------------------------------------ linear passes
 
 constexpr uint32_t LIN_NL = 2048; // limbs per CTA

@@ -718,10 +718,11 @@ uint64_t bits_of(const uint64_t *a, size_t n) {
 static const long double kLog2Phi = 0.6942419136306174017387902668985552L;
 static const long double kLog2Sqrt5 = 1.1609640474436811739351597147446950L;
 
-// Bit length of F(m) (m >= 2): floor(m log2(phi) - log2(sqrt 5)) + 1, since
+// Bit length of F(m) (F(1) = F(2) = 1; else floor(m log2(phi) - log2(sqrt 5)) + 1), since
 // F(m) = round(phi^m / sqrt 5).  When the value sits too close to an integer
 // for long double to decide, one more bit is returned (a safe upper bound).
 static uint64_t fib_bits(uint64_t m) {
+    if (m == 1 || m == 2) return 1;
     long double x = (long double)m * kLog2Phi - kLog2Sqrt5, f = floorl(x);
     uint64_t b = (uint64_t)f + 1;
     if (x - f < 1e-7L || f + 1 - x < 1e-7L) b++;
@@ -771,7 +772,32 @@ static int chain_body(uint64_t n, int i0, uint64_t *fk, uint64_t *fkm1, uint64_t
     uint64_t k = n >> i0;
     int kodd = (int)(k & 1);
     uint64_t nk, nkm1;
-    for (int i = i0 - 1; i >= 1; i--) {
+    int i = i0 - 1;
+    // the shortest steps, in one launch
+    ChainSteps S{};
+    S.nk = bk ? (uint32_t)((bk + 63) / 64) : 1, S.nkm1 = bkm1 ? (uint32_t)((bkm1 + 63) / 64) : 1;
+    S.fk = fk, S.fkm1 = fkm1, S.odd = (uint32_t)kodd;
+    for (; i >= 1 && bk <= 64 * STEP_IN && bkm1 <= bk && S.steps < FFG_CHAIN_STEPS; i--) {
+        ffg_plan pl;
+        int rc = plan_select(bk, bk, 1, &pl); // what no plan takes is refused here too
+        if (rc) return rc;
+        const uint32_t bit = (uint32_t)((n >> i) & 1);
+        k = 2 * k + bit;
+        kodd = (int)bit;
+        bk = fib_bits(k);
+        bkm1 = fib_bits(k - 1);
+        S.bits |= bit << S.steps;
+        S.n_out[S.steps++] = (uint32_t)((bk + 63) / 64);
+    }
+    if (S.steps) {
+        const uint64_t len = S.n_out[S.steps - 1];
+        ALLOC(pair, uint64_t, 2 * len);
+        S.okm1 = pair, S.ok = pair + len;
+        cudaError_t e = launch_chain_steps(S, st);
+        if (e) return fail(FFG_E_CUDA, "chain steps: %s", cudaGetErrorString(e));
+        fkm1 = S.okm1, fk = S.ok;
+    }
+    for (; i >= 1; i--) {
         const int bit = (int)((n >> i) & 1);
         if (bkm1 == 0) bkm1 = 1;
         nk = (bk + 63) / 64, nkm1 = (bkm1 + 63) / 64;
