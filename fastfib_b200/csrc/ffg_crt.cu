@@ -965,16 +965,19 @@ cudaError_t launch_school_pair(const SchoolJob *jobs, uint32_t count, cudaStream
 
 // k_school_sq_pair: the doubling step's two short squarings (operands of up
 // to a few hundred limbs) spread over more CTAs than k_school_pair gives
-// them: SQ_NL = 64 output limbs per CTA, 4 threads per column, and the
-// symmetry of a square: column j = 2 sum_{i < j - i} a_i a_(j-i) + a_(j/2)^2
-// (j even).  The same 192-bit column sums, ripple settle and last-CTA carry
-// settle as k_school.
-constexpr uint32_t SQ_NL = 64;
-constexpr uint32_t SQ_TPC = 4; // threads per column
+// them: SQ_NL = 32 output limbs per CTA, 14 threads per column (35 columns with the
+// three below), and the symmetry of a square: column j = 2 sum_{i < j - i}
+// a_i a_(j-i) + a_(j/2)^2 (j even).  The same 192-bit column sums, ripple settle and
+// last-CTA carry settle as k_school.  The time is one thread's chain of products: with
+// 64 limbs and 4 threads a column the chain of F(200 000) takes 74.4 us, with 64 and 7
+// 67.3, with 32 and 7 67.6, with 32 and 14 65.7 (F(10^6) 143 -> 131).
+constexpr uint32_t SQ_NL = 32;
+constexpr uint32_t SQ_TPC = 14; // threads per column
+constexpr uint32_t SQ_THREADS = 512;
 
 __host__ __device__ uint32_t school_sq_ctas(uint64_t nlimbs) { return (uint32_t)((nlimbs + SQ_NL - 1) / SQ_NL); }
 
-__global__ void __launch_bounds__(SCHOOL_THREADS) k_school_sq_pair(SchoolPair Pr) {
+__global__ void __launch_bounds__(SQ_THREADS) k_school_sq_pair(SchoolPair Pr) {
     after_previous();
     const SchoolJob &J = blockIdx.y ? Pr.j[1] : Pr.j[0];
     const uint32_t ncta = school_sq_ctas(J.nlimbs);
@@ -1074,7 +1077,7 @@ cudaError_t launch_school_sq_pair(const SchoolJob *jobs, uint32_t count, cudaStr
         bytes += 8.0 * (double)(jobs[i].na + jobs[i].nlimbs);
     }
     prof_begin(PK_SCHOOL, st);
-    launch_after(k_school_sq_pair, dim3(mx, count), SCHOOL_THREADS, 0, st, P);
+    launch_after(k_school_sq_pair, dim3(mx, count), SQ_THREADS, 0, st, P);
     prof_end(PK_SCHOOL, st, bytes);
     return cudaGetLastError();
 }
@@ -1235,8 +1238,11 @@ cudaError_t launch_chain_steps(const ChainSteps &J, cudaStream_t st) {
 
 // ------------------------------------------------------------ linear passes
 
-constexpr uint32_t LIN_NL = 2048; // limbs per CTA
-constexpr uint32_t LIN_THREADS = 256;
+// Two limbs a thread: the chain's short passes are one thread's latency (with 2048 limbs
+// and 256 threads a CTA the F(10^5) chain takes 47.5 us, with 1024 and 512 44.9, with 512
+// and 512, one limb a thread and twice the carries between CTAs, 49.2).
+constexpr uint32_t LIN_NL = 1024; // limbs per CTA
+constexpr uint32_t LIN_THREADS = 512;
 
 uint32_t lin_ctas(uint64_t len) { return (uint32_t)((len + LIN_NL - 1) / LIN_NL); }
 

@@ -29,10 +29,10 @@ static const uint32_t kSmallMaxL = 4096;  // one-CTA transform up to this length
 static const int kR3TabLg = 13;           // radix-3 tables cover R = 3 2^n, n < 13
 // Doubling steps whose operands have at most this many limbs square by
 // schoolbook (k_school_sq_pair, one launch for the pair) instead of the NTT
-// (transform + CRT): at these sizes both are latency-bound.  Measured on the
-// F(10^8) chain: 256 limbs 0.947 ms, 512 0.939, 768 0.939 (and 8 us less
-// than 256 on chains of n ~ 10^5).
-static const uint64_t kChainSchoolLimbs = 768;
+// (transform + CRT): at these sizes both are latency-bound.  Chain of F(10^8) with
+// limits of 512, 768, 1100 and 1536 limbs: 624, 609, 598, 598 us; of F(10^6): 132, 131,
+// 132, 127.
+static const uint64_t kChainSchoolLimbs = 1536;
 
 // ------------------------------------------------------------ host modmath
 
