@@ -903,13 +903,6 @@ __global__ void __launch_bounds__(SCHOOL_THREADS) k_school(const SchoolJob *__re
 struct SchoolPair {
     SchoolJob j[2];
 };
-__global__ void __launch_bounds__(SCHOOL_THREADS) k_school_pair(SchoolPair P) {
-    after_previous();
-    const SchoolJob &J = P.j[blockIdx.y];
-    if (blockIdx.x >= school_ctas(J.nlimbs)) return;
-    school_block(J);
-}
-
 FFG_DEV_INLINE void school_block(const SchoolJob &J) {
     constexpr uint32_t NC = SCHOOL_NL + 3; // columns j0 - 3 .. j0 + NL - 1
     __shared__ uint64_t t0s[NC], t1s[NC];
@@ -948,24 +941,8 @@ FFG_DEV_INLINE void school_block(const SchoolJob &J) {
     }
 }
 
-cudaError_t launch_school_pair(const SchoolJob *jobs, uint32_t count, cudaStream_t st) {
-    SchoolPair P{};
-    uint32_t mx = 0;
-    double bytes = 0;
-    for (uint32_t i = 0; i < count && i < 2; i++) {
-        P.j[i] = jobs[i];
-        mx = max(mx, school_ctas(jobs[i].nlimbs));
-        bytes += 8.0 * (double)(jobs[i].na + jobs[i].nb + jobs[i].nlimbs);
-    }
-    prof_begin(PK_SCHOOL, st);
-    launch_after(k_school_pair, dim3(mx, count), SCHOOL_THREADS, 0, st, P);
-    prof_end(PK_SCHOOL, st, bytes);
-    return cudaGetLastError();
-}
-
 // k_school_sq_pair: the doubling step's two short squarings (operands of up
-// to a few hundred limbs) spread over more CTAs than k_school_pair gives
-// them: SQ_NL = 32 output limbs per CTA, 14 threads per column (35 columns with the
+// to 1536 limbs) spread over more CTAs than k_school gives them: SQ_NL = 32 output limbs per CTA, 14 threads per column (35 columns with the
 // three below), and the symmetry of a square: column j = 2 sum_{i < j - i}
 // a_i a_(j-i) + a_(j/2)^2 (j even).  The same 192-bit column sums, ripple settle and
 // last-CTA carry settle as k_school.  The time is one thread's chain of products: with

@@ -236,9 +236,6 @@ __host__ __device__ uint32_t school_ctas(uint64_t nlimbs); // CTAs (and carry ma
 // count + 1 prefix sums of the jobs' crt_ctas.
 cudaError_t launch_crt_flat(const CrtJob *d_jobs, const uint32_t *d_first, uint32_t count, uint32_t total_ctas,
                             cudaStream_t st, double bytes);
-cudaError_t launch_school_pair(const SchoolJob *jobs, uint32_t count, cudaStream_t st);
-// The doubling step's two short squarings (a == b), SQ_NL output limbs per
-// CTA: school_sq_ctas(nlimbs) words of maps each.
 // Doubling steps from the pair (F(k-1), F(k)), all in one launch (k_chain_steps): at
 // most FFG_CHAIN_STEPS, on at most STEP_IN limbs each.
 constexpr int FFG_CHAIN_STEPS = 8;
@@ -251,6 +248,8 @@ struct ChainSteps {
     uint32_t n_out[FFG_CHAIN_STEPS]; // limbs of the pair after each step
 };
 cudaError_t launch_chain_steps(const ChainSteps &J, cudaStream_t st);
+// The doubling step's two short squarings (a == b), SQ_NL output limbs per
+// CTA: school_sq_ctas(nlimbs) words of maps each.
 cudaError_t launch_school_sq_pair(const SchoolJob *jobs, uint32_t count, cudaStream_t st);
 __host__ __device__ uint32_t school_sq_ctas(uint64_t nlimbs); // 1 or 2, by value
 cudaError_t launch_school_batch(const SchoolJob *d_jobs, uint32_t count, uint32_t max_ctas, cudaStream_t st,
