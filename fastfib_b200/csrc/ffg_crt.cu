@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(CRT_THREADS) k_crt_narrow(GarnerConst K, CrtJo
         const bool in = t4 < nvec && gi >= 0 && (uint64_t)gi < J.conv;
 #pragma unroll
         for (int k = 0; k < 3; k++)
-            rv[v][k] = in ? __ldg((const uint4 *)(J.y + k * J.y_stride + gi)) : make_uint4(0, 0, 0, 0);
+            rv[v][k] = in ? *(const uint4 *)(J.y + k * J.y_stride + gi) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int v = 0; v < VPT; v++) {
@@ -879,7 +879,7 @@ FFG_DEV_INLINE void school_col(const SchoolJob &J, int64_t j, uint64_t &t0, uint
     const int64_t ns = (int64_t)(a_short ? J.na : J.nb), nl = (int64_t)(a_short ? J.nb : J.na);
     const int64_t i0 = j - nl + 1 > 0 ? j - nl + 1 : 0, i1 = j < ns - 1 ? j : ns - 1;
     for (int64_t i = i0; i <= i1; i++) {
-        const u128 pr = (u128)__ldg(&S[i]) * __ldg(&Lg[j - i]);
+        const u128 pr = (u128)S[i] * Lg[j - i];
         const uint64_t lo = (uint64_t)pr, hi = (uint64_t)(pr >> 64);
         t0 += lo;
         const uint64_t c0 = t0 < lo;
