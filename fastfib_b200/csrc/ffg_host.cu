@@ -17,6 +17,7 @@
 #include "ffg.h"
 #include "ffg_hostctx.h"
 #include "ffg_internal.h"
+#include "ffg_slots.h"
 
 namespace ffg {
 
@@ -980,72 +981,7 @@ int pinned_release(void *p) {
     return 0;
 }
 
-// Host copies of an entry point's operands and result, through four pinned slots in
-// turn: the CPU fills or empties one while the DMA works on the others (the driver's
-// own pageable copies wait for each other: 50001 x 48000 limbs, 1.6 MB of copies,
-// 305 -> 200 us a product; 1 000 000 x 900 000, 13 ms -> 2.8).  Made on first use,
-// freed by ffg_shutdown, used under g_mu.
-constexpr size_t kSlotBytes = 128 << 10;
-constexpr int kSlots = 4;
-static struct HostSlots {
-    char *mem = nullptr;
-    cudaEvent_t done[kSlots] = {};
-} g_slots;
-
-static void slots_free() {
-    for (auto &e : g_slots.done)
-        if (e) cudaEventDestroy(e);
-    if (g_slots.mem) cudaFreeHost(g_slots.mem);
-    g_slots = HostSlots{};
-}
-
-static int slots_ready() {
-    if (!g_slots.mem) {
-        cudaError_t e = cudaMallocHost(&g_slots.mem, kSlots * kSlotBytes);
-        for (int k = 0; k < kSlots && !e; k++) e = cudaEventCreateWithFlags(&g_slots.done[k], cudaEventDisableTiming);
-        if (e) {
-            slots_free();
-            return fail(FFG_E_NOMEM, "pinned host slots: %s", cudaGetErrorString(e));
-        }
-    }
-    return FFG_OK;
-}
-
-// Queues the copy of n bytes of src to the device; src has been read when it returns.
-static int slots_up(void *dst, const void *src, size_t n, int *turn, cudaStream_t st) {
-    for (size_t at = 0; at < n; at += kSlotBytes) {
-        const int k = (*turn)++ % kSlots;
-        const size_t len = std::min(kSlotBytes, n - at);
-        char *slot = g_slots.mem + k * kSlotBytes;
-        if (*turn > kSlots) CK(cudaEventSynchronize(g_slots.done[k]));
-        memcpy(slot, (const char *)src + at, len);
-        CK(cudaMemcpyAsync((char *)dst + at, slot, len, cudaMemcpyHostToDevice, st));
-        CK(cudaEventRecord(g_slots.done[k], st));
-    }
-    return FFG_OK;
-}
-
-// Copies n bytes from the device, queued behind all that st holds.
-static int slots_down(void *dst, const void *src, size_t n, cudaStream_t st) {
-    const size_t chunks = (n + kSlotBytes - 1) / kSlotBytes;
-    for (size_t c = 0; c < chunks + kSlots; c++) {
-        const int k = (int)(c % kSlots);
-        if (c >= kSlots) { // chunk c - kSlots has its slot until here
-            const size_t at = (c - kSlots) * kSlotBytes;
-            if (at < n) {
-                CK(cudaEventSynchronize(g_slots.done[k]));
-                memcpy((char *)dst + at, g_slots.mem + k * kSlotBytes, std::min(kSlotBytes, n - at));
-            }
-        }
-        if (c < chunks) {
-            const size_t at = c * kSlotBytes;
-            CK(cudaMemcpyAsync(g_slots.mem + k * kSlotBytes, (const char *)src + at, std::min(kSlotBytes, n - at),
-                               cudaMemcpyDeviceToHost, st));
-            CK(cudaEventRecord(g_slots.done[k], st));
-        }
-    }
-    return FFG_OK;
-}
+static HostSlots g_slots; // made on first use, freed by ffg_shutdown
 
 static bool graphs_enabled() {
     const char *e = getenv("FFG_NO_GRAPH");
@@ -1059,9 +995,7 @@ static int fib_chain(uint64_t n, int i0, const uint64_t *hkm1, size_t hnkm1, con
     const uint64_t cap0 = (std::max(nk, nkm1) + 31) & ~31ull;
     ALLOC(fk, uint64_t, 2 * cap0); // the pair in one block: one copy
     uint64_t *const fkm1 = fk + cap0;
-    if (2 * cap0 * 8 <= kSlotBytes * kSlots) {
-        int rc = slots_ready();
-        if (rc) return rc;
+    if (2 * cap0 * 8 <= HostSlots::kBytes * HostSlots::kCount && g_slots.ready()) {
         uint64_t *h = (uint64_t *)g_slots.mem;
         memset(h, 0, 2 * cap0 * 8);
         if (hnk) memcpy(h, hk, hnk * 8);
@@ -1263,10 +1197,9 @@ extern "C" int ffg_mul_host(uint64_t *out, size_t *nout, const uint64_t *a, size
     }
     const uint64_t nr = na + nb + 1;
     ALLOC(dr, uint64_t, nr);
-    if ((rc = slots_ready())) return rc;
-    int turn = 0;
-    if ((rc = slots_up(da, a, na * 8, &turn, st))) return rc;
-    if (!square && (rc = slots_up(db, b, nb * 8, &turn, st))) return rc;
+    g_slots.ready();
+    CK(g_slots.up(da, a, na * 8, st));
+    if (!square) CK(g_slots.up(db, b, nb * 8, st));
     Prod p{da, db, na, nb, ba, bb, dr, 0};
     rc = mul_one(p, square != 0, st);
     if (rc) return rc;
@@ -1275,7 +1208,7 @@ extern "C" int ffg_mul_host(uint64_t *out, size_t *nout, const uint64_t *a, size
     const uint64_t sure = (ba + bb - 1 + 63) / 64, all = (ba + bb + 63) / 64;
     uint64_t top = 0;
     if (all > sure) CK(cudaMemcpyAsync(&top, dr + sure, 8, cudaMemcpyDeviceToHost, st));
-    if ((rc = slots_down(out, dr, sure * 8, st))) return rc;
+    CK(g_slots.down(out, dr, sure * 8, st));
     CK(cudaStreamSynchronize(st));
     if (top) out[sure] = top;
     *nout = sure + (top ? 1 : 0);
@@ -1357,7 +1290,7 @@ extern "C" void ffg_shutdown(void) {
     dec_free();
     for (auto &b : g_pinned_pool) cudaFreeHost(b.first);
     g_pinned_pool.clear();
-    slots_free();
+    g_slots.release();
     cudaEventDestroy(g.ev0);
     cudaEventDestroy(g.ev1);
     cudaStreamDestroy(g.stream);
