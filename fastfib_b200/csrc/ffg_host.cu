@@ -1414,22 +1414,39 @@ static int noalloc_address(int dev, void **addr) {
     return FFG_OK;
 }
 
-// The kernels that products within that scratch launch at the geometries in
-// force (lengths up to 2^19), once.
+// The kernels that products of length 2^lg (3 2^lg) within that scratch launch at the
+// geometry in force.
+static int noalloc_length_load(uint32_t lg, uint32_t r3) {
+    ffg_plan pl{};
+    pl.lg = lg, pl.r3 = r3, pl.L = (uint64_t)(r3 ? 3 : 1) << lg;
+    gpu_geometry(&pl);
+    for (int square = 0; square < 2; square++)
+        CK(pl.kernel ? load_four_step(four_step_geometry(pl, square != 0)) : load_conv(lg, r3, square != 0));
+    return FFG_OK;
+}
+
+// All of them (lengths up to 2^19): by ffg_init, then again the length whose geometry
+// changes; a change without a context leaves them to the next ffg_init.
+static bool g_noalloc_loaded = false;
+static constexpr uint32_t kNoAllocLg[2] = {19, 17}; // by radix-3 factor
+
 static int noalloc_kernels_load() {
-    static bool done = false;
-    if (done) return FFG_OK;
+    if (g_noalloc_loaded) return FFG_OK;
     CK(crt_kernel_load());
     for (uint32_t r3 = 0; r3 < 2; r3++)
-        for (uint32_t lg = 4; lg <= (r3 ? 17u : 19u); lg++) {
-            ffg_plan pl{};
-            pl.lg = lg, pl.r3 = r3, pl.L = (uint64_t)(r3 ? 3 : 1) << lg;
-            gpu_geometry(&pl);
-            for (int square = 0; square < 2; square++)
-                CK(pl.kernel ? load_four_step(four_step_geometry(pl, square != 0)) : load_conv(lg, r3, square != 0));
+        for (uint32_t lg = 4; lg <= kNoAllocLg[r3]; lg++) {
+            const int rc = noalloc_length_load(lg, r3);
+            if (rc) return rc;
         }
-    done = true;
+    g_noalloc_loaded = true;
     return FFG_OK;
+}
+
+static int noalloc_geometry_changed(uint32_t lg, uint32_t r3) {
+    if (!g.ready) g_noalloc_loaded = false;
+    if (!g_noalloc_loaded || lg < 4 || lg > kNoAllocLg[r3]) return FFG_OK;
+    const int rc = ensure_ready(); // the context's device
+    return rc ? rc : noalloc_length_load(lg, r3);
 }
 
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -1521,7 +1538,7 @@ extern "C" int ffg_set_geometry(uint32_t lg, uint32_t r3, uint32_t row_lg, uint3
         g_geo[lg][r3] = Geo{1, (uint8_t)row_lg, (uint8_t)wc};
     }
     chain_cache_clear(); // captured chains hold launches of the old geometry
-    return FFG_OK;
+    return noalloc_geometry_changed(lg, r3);
 }
 
 extern "C" int ffg_get_geometry(uint32_t lg, uint32_t r3, uint32_t *row_lg, uint32_t *wc) {

@@ -218,7 +218,9 @@ int ffg_load_tuning(const char *path);
    per operand), or that need the split multiply, return FFG_E_RANGE with the
    bytes needed in the message.  ffg_init must have run first: it builds the
    device tables, looks the array's address up (with the device current) and
-   loads the kernels used here, so the first call allocates nothing either.
+   loads the kernels used here, so the first call allocates nothing either; a
+   geometry set after it (ffg_set_geometry, ffg_load_tuning) loads its own
+   kernels when it is set.
    All calls share the one array, and it keeps the last call's contents:
    calls whose GPU work overlaps (different streams, no ordering between
    them) race and corrupt each other's results. */
