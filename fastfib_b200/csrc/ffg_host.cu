@@ -995,12 +995,14 @@ static int fib_chain(uint64_t n, int i0, const uint64_t *hkm1, size_t hnkm1, con
     const uint64_t cap0 = (std::max(nk, nkm1) + 31) & ~31ull;
     ALLOC(fk, uint64_t, 2 * cap0); // the pair in one block: one copy
     uint64_t *const fkm1 = fk + cap0;
+    uint64_t h2d = 8 * (uint64_t)(hnk + hnkm1);
     if (2 * cap0 * 8 <= HostSlots::kBytes * HostSlots::kCount && g_slots.ready()) {
         uint64_t *h = (uint64_t *)g_slots.mem;
         memset(h, 0, 2 * cap0 * 8);
         if (hnk) memcpy(h, hk, hnk * 8);
         if (hnkm1) memcpy(h + cap0, hkm1, hnkm1 * 8);
-        CK(cudaMemcpyAsync(fk, h, 2 * cap0 * 8, cudaMemcpyHostToDevice, st));
+        h2d = 2 * cap0 * 8;
+        CK(cudaMemcpyAsync(fk, h, h2d, cudaMemcpyHostToDevice, st));
     } else {
         CK(cudaMemsetAsync(fk, 0, 2 * cap0 * 8, st));
         CK(cudaMemcpyAsync(fk, hk, hnk * 8, cudaMemcpyHostToDevice, st));
@@ -1104,7 +1106,7 @@ copy_back:
     float ms = 0;
     cudaEventElapsedTime(&ms, g.ev0, g.ev1);
     g.chain_ms = ms;
-    g.chain_h2d = 8 * (uint64_t)(hnk + hnkm1);
+    g.chain_h2d = h2d;
     g.chain_d2h = 8 * nres;
     while (nres > 1 && h[nres - 1] == 0) nres--;
     *out = h;
