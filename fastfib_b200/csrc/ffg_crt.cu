@@ -187,7 +187,9 @@ template <int T, int SL, int B> struct CrtGeo {
     static constexpr uint32_t ROW = SL + 4, PLANE = T * ROW;
     static_assert(SL * B % 32 == 0 && W <= (int)ROW && W >= 8 && SL >= 8 && T % 32 == 0, "whole words");
 };
-// The shortest super-limbs of a width (short products: the sums' serial chain).
+// The shortest super-limbs of a width (the sums' serial chain).  The doubling step's
+// fused CRT gains by them (chain of F(10^8) 633 us, with super-limbs of 32 644); a plain
+// short product does not (300, 1000 and 65536 limbs equal within noise) and shares them.
 template <int B> struct CrtShort {
     static constexpr int SL = B == 32 ? 8 : (B == 34 ? 16 : 32);
 };
@@ -594,8 +596,9 @@ __global__ void __launch_bounds__(crt_threads<F>(), F == CF_BATCH ? 6 : (F == CF
     crt_any<F>(K, J, blockIdx.x);
 }
 
-// Up to two CRTs by value (the doubling step's two squarings): product
-// blockIdx.y, its CTA blockIdx.x.
+// Two CRTs by value, product blockIdx.y, its CTA blockIdx.x: the doubling step's two
+// squarings when its linear pass is a launch of its own (FFG_NO_CRT_LIN=1, the
+// comparison with k_crt_lin).
 struct CrtPair {
     CrtJob j[2];
 };
@@ -942,9 +945,9 @@ FFG_DEV_INLINE void school_block(const SchoolJob &J) {
 }
 
 // k_school_sq_pair: the doubling step's two short squarings (operands of up
-// to 1536 limbs) spread over more CTAs than k_school gives them: SQ_NL = 32 output limbs per CTA, 14 threads per column (35 columns with the
-// three below), and the symmetry of a square: column j = 2 sum_{i < j - i}
-// a_i a_(j-i) + a_(j/2)^2 (j even).  The same 192-bit column sums, ripple settle and
+// to 1536 limbs) spread over more CTAs than k_school gives them: SQ_NL = 32 output
+// limbs per CTA, 14 threads per column (35 columns with the three below), and the
+// symmetry of a square: column j = 2 sum_{i < j - i} a_i a_(j-i) + a_(j/2)^2 (j even).  The same 192-bit column sums, ripple settle and
 // last-CTA carry settle as k_school.  The time is one thread's chain of products: with
 // 64 limbs and 4 threads a column the chain of F(200 000) takes 74.4 us, with 64 and 7
 // 67.3, with 32 and 7 67.6, with 32 and 14 65.7 (F(10^6) 143 -> 131).
